@@ -3,6 +3,7 @@
 #include <cstring>
 #include <type_traits>
 #include "mg.cuh"
+#include "mg_tail.cuh"
 
 namespace incrmt {
 
@@ -776,156 +777,6 @@ __global__ void k_coarse_inverse(const double *st, int m, int n, int px, int py,
     }
 }
 
-/** Coarsest solve by the dense inverse: z = G b. */
-template <class T>
-__device__ __forceinline__ void coarse_direct(const T *G, const T *b, T *z, int N) {
-    for (int r = threadIdx.x; r < N; r += blockDim.x) {
-        T t = 0;
-        for (int q = 0; q < N; q++) t += G[static_cast<long>(r) * N + q] * b[q];
-        z[r] = t;
-    }
-}
-
-template <class T>
-__global__ void k_coarse_direct(const T *G, const T *b, T *z, int N) {
-    coarse_direct(G, b, z, N);
-}
-
-/** Levels handled by the one-block tail kernel. */
-constexpr int kTailMaxLevels = 12;
-constexpr int kTailMaxSize = 1024;  // unknowns of the first tail level at most
-constexpr size_t kTailSmemBudget = 160 * 1024;  // shared memory for the smallest tail levels
-
-template <class T>
-struct TailLevels {
-    int first, count, px, py;
-    const double *P[kTailMaxLevels]; // prolongation weights of each tail level but the last
-    int smem_from;                 // levels >= smem_from live in shared memory
-    const T *ginv;                 // dense inverse of the coarsest level, or null
-    long smem_off[kTailMaxLevels]; // element offsets of st, then z, then b
-    int m[kTailMaxLevels], n[kTailMaxLevels];
-    long N[kTailMaxLevels];
-    bool kx[kTailMaxLevels], ky[kTailMaxLevels];
-    T *z[kTailMaxLevels];
-    T *b[kTailMaxLevels];
-    const T *st[kTailMaxLevels];
-};
-
-template <class T>
-__device__ __forceinline__ GenOp<T> tail_op(const TailLevels<T> &L, int l) {
-    GenOp<T> g; g.m = L.m[l]; g.n = L.n[l]; g.px = L.px; g.py = L.py; g.N = L.N[l]; g.st = L.st[l];
-    return g;
-}
-
-/** Smoothing of one tail level. Levels of at most kWarpLevel unknowns are
- * swept by the first warp alone with warp barriers (a block barrier per
- * colour phase would dominate there); the block waits once at the end. */
-constexpr int kWarpLevel = 256;
-
-template <class T>
-__device__ void tail_smooth(const TailLevels<T> &L, int l, int sweeps) {
-    const int pis[4] = {0, 1, 1, 0}, pjs[4] = {0, 1, 0, 1};
-    const GenOp<T> op = tail_op(L, l);
-    const int m = L.m[l], n = L.n[l];
-    T *z = L.z[l];
-    const T *b = L.b[l];
-    const bool warp_only = m * n <= kWarpLevel;
-    if (warp_only && threadIdx.x >= 32) { __syncthreads(); return; }
-    const int nth = warp_only ? 32 : blockDim.x;
-    for (int s = 0; s < sweeps; s++)
-        for (int c = 0; c < 4; c++) {
-            const int mc = (m - pis[c] + 1) / 2, nc = (n - pjs[c] + 1) / 2;
-            for (int p = threadIdx.x; p < mc * nc; p += nth) {
-                const int i = 2 * (p % mc) + pis[c], j = 2 * (p / mc) + pjs[c];
-                z[i + m * j] = gs_update(op, i, j, z, b[i + m * j]);
-            }
-            if (warp_only) __syncwarp();
-            else __syncthreads();
-        }
-    if (warp_only) __syncthreads();
-}
-
-/** The V-cycle below (and including) level L.first in one block: smoothing,
- * restriction and prolongation of every tail level with block barriers
- * between phases, and the coarsest solve. The levels are small enough to sit
- * in L2, so the cost is the barriers rather than launches. */
-template <class T>
-__global__ void __launch_bounds__(1024) k_tail(TailLevels<T> Lp, int nu1, int nu2, int coarse_sweeps) {
-    // The smallest levels are moved into shared memory: stencils copied in,
-    // iterate and right-hand side written there by the restriction.
-    extern __shared__ __align__(16) unsigned char tail_smem[];
-    T *sbase = reinterpret_cast<T *>(tail_smem);
-    TailLevels<T> L = Lp;
-    for (int l = L.smem_from; l < L.count; l++) {
-        T *st = sbase + L.smem_off[l];
-        const long n9 = 9 * L.N[l];
-        for (long q = threadIdx.x; q < n9; q += blockDim.x) st[q] = L.st[l][q];
-        if (l == 0) {
-            // the first tail level's right-hand side and iterate come from the
-            // restriction before the tail; its iterate goes back at the end
-            for (long q = threadIdx.x; q < L.N[0]; q += blockDim.x) {
-                st[n9 + q] = L.z[0][q];
-                st[n9 + L.N[0] + q] = L.b[0][q];
-            }
-        }
-        L.st[l] = st;
-        L.z[l] = st + n9;
-        L.b[l] = st + n9 + L.N[l];
-    }
-    __syncthreads();
-    const int last = L.count - 1;
-    for (int l = 0; l < last; l++) {
-        tail_smooth(L, l, nu1);
-        const GenOp<T> op = tail_op(L, l);
-        const int fm = L.m[l], fn = L.n[l], cm = L.m[l + 1], cn = L.n[l + 1];
-        const bool kx = L.kx[l], ky = L.ky[l];
-        for (int q = threadIdx.x; q < cm * cn; q += blockDim.x) {
-            const int I = q % cm, J = q / cm;
-            const int x0 = kx ? 2 * I - 1 : I, x1 = kx ? 2 * I + 1 : I, y0 = ky ? 2 * J - 1 : J,
-                      y1 = ky ? 2 * J + 1 : J;
-            T t = 0;
-            for (int fj = y0; fj <= y1; fj++)
-                for (int fi = x0; fi <= x1; fi++) {
-                    const T w = static_cast<T>(pweight(L.P[l], fm, fn, L.px, L.py, kx, ky, fi, fj, I, J));
-                    if (w == 0) continue;
-                    bool ok = true;
-                    const int i = wrap_idx(fi, fm, L.px, ok), j = wrap_idx(fj, fn, L.py, ok);
-                    const int f = i + fm * j;
-                    t = add_prod(t, w, residual_at(op, i, j, static_cast<const T *>(L.z[l]), L.b[l][f]));
-                }
-            L.b[l + 1][q] = t;
-            L.z[l + 1][q] = 0;
-        }
-        __syncthreads();
-    }
-    if (L.ginv) {
-        coarse_direct(L.ginv, L.b[last], L.z[last], static_cast<int>(L.N[last]));
-        __syncthreads();
-    } else {
-        tail_smooth(L, last, coarse_sweeps);
-    }
-    for (int l = last - 1; l >= 0; l--) {
-        const int fm = L.m[l], fn = L.n[l], cm = L.m[l + 1], cn = L.n[l + 1];
-        for (int q = threadIdx.x; q < fm * fn; q += blockDim.x) {
-            const int i = q % fm, j = q / fm;
-            const double *w = L.P[l] + 4 * static_cast<long>(q);
-            const int bx = base_of(i, L.kx[l]), by = base_of(j, L.ky[l]);
-            T t = 0;
-            for (int r = 0; r < 4; r++) {
-                if (w[r] == 0) continue;
-                const int I = corner_of(bx, r & 1, cm, L.px, L.kx[l]), J = corner_of(by, r >> 1, cn, L.py, L.ky[l]);
-                if (I < 0 || J < 0) continue;
-                t = add_prod(t, static_cast<T>(w[r]), L.z[l + 1][I + cm * J]);
-            }
-            L.z[l][q] += t;
-        }
-        __syncthreads();
-        tail_smooth(L, l, nu2);
-    }
-    if (L.smem_from == 0)
-        for (long q = threadIdx.x; q < L.N[0]; q += blockDim.x) Lp.z[0][q] = L.z[0][q];
-}
-
 /** FP64 residual r = b - A z, optionally stored in FP32, with per-block sums
  * of r^2 in partial[blockIdx.x]. Each block takes every gridDim.x-th row,
  * its threads the row's unknowns (coalesced, no index division). */
@@ -1149,6 +1000,15 @@ constexpr int kRedBlocks = 4 * kB200SMs;  // reduction grid: 4 x 148 blocks of 2
 inline dim3 grid2(int m, int n) { return dim3(cdiv(m, 32), cdiv(n, 8)); }
 const dim3 kBlk2(32, 8);
 
+/** The attributes a launch of k_tail needs. */
+template <class T, bool SEQ>
+cudaError_t set_tail_attr() {
+    const cudaError_t e = cudaFuncSetAttribute(k_tail<T, SEQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(kTailSmemBudget));
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(k_tail<T, SEQ>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+}
+
 /** Runs `sweeps` four-colour sweeps on the iterate z. Two sweeps on a grid
  * whose periodic directions have even sizes run as one tile-fused launch that
  * reads z and writes zalt (*res = zalt); otherwise one launch per colour
@@ -1333,24 +1193,19 @@ int Multigrid::build_hierarchy() {
         INCRMT_CK(cudaFuncSetAttribute(k_coarse_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(sizeof(double) * (2 * kDirectMax * kDirectMax + kDirectMax))));
     }
-    INCRMT_CK(cudaFuncSetAttribute(k_tail<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(kTailSmemBudget)));
+    INCRMT_CK((set_tail_attr<double, false>()));
+    INCRMT_CK((set_tail_attr<double, true>()));
+    INCRMT_CK((set_tail_attr<float, false>()));
+    INCRMT_CK((set_tail_attr<float, true>()));
     INCRMT_CK(cudaFuncSetAttribute(k_smooth_tile_gen<double, 2, 16, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    gen_tile_smem<double>()));
     INCRMT_CK(cudaFuncSetAttribute(k_smooth_tile_gen<float, 2, 16, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    gen_tile_smem<float>()));
-    INCRMT_CK(cudaFuncSetAttribute(k_tail<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(kTailSmemBudget)));
-
     const int gal_smem = static_cast<int>(galerkin_tile_smem(true, true));
     INCRMT_CK(set_galerkin_attr<MacOp<double>>(gal_smem));
     INCRMT_CK(set_galerkin_attr<FemOp<double>>(gal_smem));
     INCRMT_CK(set_galerkin_attr<GenOp<double>>(gal_smem));
-    // First level small enough for the one-block tail kernel (never level 0).
-    tail_level = -1;
-    for (int l = 1; l < static_cast<int>(lev.size()); l++)
-        if (lev[l].N <= kTailMaxSize && static_cast<int>(lev.size()) - l <= kTailMaxLevels) { tail_level = l; break; }
-    return INCRMT_OK;
+    return choose_tail();
 }
 
 void Multigrid::destroy() {
@@ -1362,6 +1217,7 @@ void Multigrid::destroy() {
     cudaFree(ex); cudaFree(ey); cudaFree(exf); cudaFree(eyf); cudaFree(c); cudaFree(cf);
     cudaFree(rho); cudaFree(bbuf); cudaFree(zbuf); cudaFree(partial); cudaFree(dnorm);
     cudaFree(ginv); cudaFree(ginvf); ginv = nullptr; ginvf = nullptr;
+    cudaFree(tail_pk); tail_pk = nullptr;
 
     if (hnorm) cudaFreeHost(hnorm);
     if (gexec) { cudaGraphExecDestroy(gexec); gexec = nullptr; }
@@ -1496,7 +1352,7 @@ int Multigrid::galerkin_all() {
         launches++;
         INCRMT_CKL("k_coarse_inverse");
     }
-    return INCRMT_OK;
+    return tail_pack<double>();
 }
 
 int Multigrid::galerkin_graph() {
@@ -1536,6 +1392,8 @@ int Multigrid::cast_levels() {
         launches++;
     }
     INCRMT_CKL("k_cast_stencil");
+    int r = tail_pack<float>();
+    if (r) return r;
     f32_stale = false;
     return INCRMT_OK;
 }
@@ -1551,8 +1409,7 @@ int Multigrid::cycle64(int l, const double *b0, double *z0) {
         if (l == 0) {
             if (sys == INCRMT_SYS_MAC) k_coarse<<<1, 256, 0, stream>>>(mac64(), z, b, L.m, L.n, kCoarseSweeps);
             else k_coarse<<<1, 256, 0, stream>>>(fem64(), z, b, L.m, L.n, kCoarseSweeps);
-        } else if (ginv) k_coarse_direct<double><<<1, 256, 0, stream>>>(ginv, b, z, static_cast<int>(L.N));
-        else k_coarse<<<1, 256, 0, stream>>>(g, z, b, L.m, L.n, kCoarseSweeps);
+        } else k_coarse<<<1, 256, 0, stream>>>(g, z, b, L.m, L.n, kCoarseSweeps);
         launches++;
         INCRMT_CKL("k_coarse");
         return INCRMT_OK;
@@ -1644,8 +1501,7 @@ int Multigrid::cycle32(int l) {
         if (l == 0) {
             if (sys == INCRMT_SYS_MAC) k_coarse<<<1, 256, 0, stream>>>(mac32(), z, b, L.m, L.n, kCoarseSweeps);
             else k_coarse<<<1, 256, 0, stream>>>(fem32(), z, b, L.m, L.n, kCoarseSweeps);
-        } else if (ginvf) k_coarse_direct<float><<<1, 256, 0, stream>>>(ginvf, b, z, static_cast<int>(L.N));
-        else k_coarse<<<1, 256, 0, stream>>>(g, z, b, L.m, L.n, kCoarseSweeps);
+        } else k_coarse<<<1, 256, 0, stream>>>(g, z, b, L.m, L.n, kCoarseSweeps);
         launches++;
         INCRMT_CKL("k_coarse");
         return INCRMT_OK;
@@ -1682,55 +1538,186 @@ int Multigrid::cycle32(int l) {
     return INCRMT_OK;
 }
 
-/** Shared-memory layout of the tail: the coarsest levels, from the bottom
- * up, while their stencils, iterates and right-hand sides fit in the budget.
- * \return the dynamic shared memory in bytes. */
+namespace {
+
+/** The tail's plan from level `first` down (see mg_tail.cuh), over at most
+ * max_blocks blocks; false if some level does not fit. Levels of more than
+ * kTailRoot cells are cut into strips over the cluster. */
 template <class T>
-size_t tail_layout(TailLevels<T> &L, size_t budget) {
-    long off = 0;
-    L.smem_from = L.count;
-    for (int k = L.count - 1; k >= 0; k--) {
-        const long need = 11 * L.N[k];
-        if (static_cast<size_t>(off + need) * sizeof(T) > budget) break;
-        L.smem_from = k;
-        off += need;
+bool tail_plan(const std::vector<MgLevel> &lev, int first, int px, int py, const T *ginv, int max_blocks,
+               TailPlan<T> &p, int &blocks, int &threads, size_t &smem) {
+    p = TailPlan<T>{};
+    p.count = static_cast<int>(lev.size()) - first;
+    if (p.count < 1 || p.count > kTailMaxLevels) return false;
+    p.px = px; p.py = py; p.nu1 = kNu1; p.nu2 = kNu2; p.coarse_sweeps = kCoarseSweeps;
+    p.ginv = ginv;
+    for (int k = 0; k < p.count; k++) {
+        const MgLevel &L = lev[first + k];
+        TailLevel<T> &t = p.lev[k];
+        t.m = L.m; t.n = L.n; t.cx = (L.m + 1) / 2; t.cy = (L.n + 1) / 2;
+        t.kx = L.kx; t.ky = L.ky;
+        if constexpr (sizeof(T) == 8) t.pk = L.pk;
+        else t.pk = L.pkf;
+        t.seq = px && L.m % 2 ? 2 : (py && L.n % 2 ? 1 : 0);
+        t.dist = static_cast<long>(t.cx) * t.cy > kTailRoot;
+        t.rows = t.cy;
+        if (t.dist && (t.seq || k == p.count - 1)) return false;
+        if (t.dist) p.ndist = k + 1;
     }
+    // A strip's cell rows halve with the level, so the first level's are a
+    // multiple of 2 for every such step between strip levels.
+    blocks = 1;
+    if (p.ndist) {
+        int step = 1;
+        for (int k = 0; k + 1 < p.ndist; k++)
+            if (p.lev[k].ky) step *= 2;
+        int rows = cdiv(cdiv(p.lev[0].cy, max_blocks), step) * step;
+        blocks = cdiv(p.lev[0].cy, rows);
+        for (int k = 0; k < p.ndist; k++) {
+            p.lev[k].rows = rows;
+            if (static_cast<long>(rows) * p.lev[k].cx > kTailThreads) return false;
+            if (p.lev[k].ky) rows /= 2;
+        }
+    }
+    threads = 96;  // the coarsest solve's rows
     long o = 0;
-    for (int k = L.smem_from; k < L.count; k++) { L.smem_off[k] = o; o += 11 * L.N[k]; }
-    return static_cast<size_t>(o) * sizeof(T);
+    for (int k = 0; k < p.count; k++) {
+        TailLevel<T> &t = p.lev[k];
+        if (t.rows * t.cx > threads) threads = t.rows * t.cx;
+        t.used = cdiv(t.cy, t.rows);
+        t.mul = ((1 << 20) + t.cx - 1) / t.cx;
+        const long za = 4L * (t.rows + 1) * (t.cx + 2);
+        t.zo = static_cast<int>(o); o += za;
+        t.ro = static_cast<int>(o); o += k < p.count - 1 ? za : 0;
+        t.bo = static_cast<int>(o); o += k ? 4L * t.rows * t.cx : 0;
+    }
+    threads = (threads + 31) / 32 * 32;
+    p.zeroed = static_cast<int>(o);
+    const long budget = static_cast<long>(kTailSmemBudget / sizeof(T));
+    if (o > budget) return false;
+    p.go = -1;
+    const long Nc = lev.back().N;
+    if (ginv) {
+        if (o + Nc * Nc > budget) return false;
+        p.go = static_cast<int>(o);
+        o += Nc * Nc;
+    }
+    // Staged from the coarsest level up while they fit: all slots, else the
+    // stencils alone.
+    for (int k = p.count - 1; k >= 0; k--) {
+        if (k == p.count - 1 && ginv) continue;  // solved by the inverse alone
+        const long np = static_cast<long>(p.lev[k].rows) * p.lev[k].cx;
+        int slots = kTailSlots<T>;
+        if (o + slots * np > budget) slots = kTailRw<T>;
+        if (o + slots * np > budget) break;
+        p.lev[k].co = static_cast<int>(o);
+        p.lev[k].staged = slots;
+        o += slots * np;
+    }
+    smem = static_cast<size_t>(o) * sizeof(T);
+    return true;
 }
 
-int Multigrid::tail64() {
-    TailLevels<double> T{};
-    T.first = tail_level; T.count = static_cast<int>(lev.size()) - tail_level; T.px = px; T.py = py;
-    for (int k = 0; k < T.count; k++) {
-        const MgLevel &L = lev[tail_level + k];
-        T.m[k] = L.m; T.n[k] = L.n; T.N[k] = L.N; T.kx[k] = L.kx; T.ky[k] = L.ky;
-        T.z[k] = L.z; T.b[k] = L.b; T.st[k] = L.st; T.P[k] = L.P;
+cudaLaunchConfig_t tail_config(int blocks, int threads, size_t smem, cudaStream_t s, cudaLaunchAttribute *at) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(blocks);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = blocks;
+    at->val.clusterDim.y = at->val.clusterDim.z = 1;
+    c.attrs = at;
+    c.numAttrs = 1;
+    return c;
+}
+
+}  // namespace
+
+int Multigrid::choose_tail() {
+    // The first level (never level 0) from which on everything fits, at the
+    // largest cluster size that the device grants.
+    tail_level = -1;
+    for (int mb = kTailBlocks; mb >= 1 && tail_level < 0; mb /= 2)
+        for (int l = 1; l < static_cast<int>(lev.size()); l++) {
+            TailPlan<double> p;
+            int blocks, threads;
+            size_t smem;
+            if (!tail_plan<double>(lev, l, px, py, ginv, mb, p, blocks, threads, smem)) continue;
+            cudaLaunchAttribute at[1];
+            cudaLaunchConfig_t c = tail_config(blocks, threads, smem, stream, at);
+            int active = 0;
+            if (cudaOccupancyMaxActiveClusters(&active, k_tail<double, true>, &c) != cudaSuccess) cudaGetLastError();
+            if (active < 1) break;
+            tail_level = l;
+            tail_max_blocks = mb;
+            break;
+        }
+    if (tail_level < 0) return INCRMT_OK;
+    auto cells = [](const MgLevel &L) { return static_cast<size_t>((L.m + 1) / 2) * ((L.n + 1) / 2); };
+    size_t total = 0;
+    for (size_t l = tail_level; l < lev.size(); l++) total += cells(lev[l]);
+    INCRMT_CK(cudaMalloc(&tail_pk, (sizeof(double) * kTailSlots<double> + sizeof(float) * kTailSlots<float>) * total));
+    double *d = static_cast<double *>(tail_pk);
+    float *f = reinterpret_cast<float *>(d + kTailSlots<double> * total);
+    for (size_t l = tail_level; l < lev.size(); l++) {
+        lev[l].pk = d;
+        lev[l].pkf = f;
+        d += kTailSlots<double> * cells(lev[l]);
+        f += kTailSlots<float> * cells(lev[l]);
     }
-    T.ginv = ginv;
-    const size_t sm = tail_layout(T, kTailSmemBudget);
-    k_tail<double><<<1, 1024, sm, stream>>>(T, kNu1, kNu2, kCoarseSweeps);
+    return INCRMT_OK;
+}
+
+template <class T>
+int Multigrid::tail_pack() {
+    if (tail_level < 0) return INCRMT_OK;
+    TailPack<T> p{};
+    p.count = static_cast<int>(lev.size()) - tail_level;
+    p.px = px; p.py = py;
+    int most = 0;
+    for (int k = 0; k < p.count; k++) {
+        const MgLevel &L = lev[tail_level + k];
+        TailPackLevel<T> &t = p.lev[k];
+        t.m = L.m; t.n = L.n; t.kx = L.kx; t.ky = L.ky; t.P = L.P;
+        t.cells = ((L.m + 1) / 2) * ((L.n + 1) / 2);
+        if constexpr (sizeof(T) == 8) { t.st = L.st; t.pk = L.pk; }
+        else { t.st = L.stf; t.pk = L.pkf; }
+        if (t.cells > most) most = t.cells;
+    }
+    k_tail_pack<T><<<dim3(cdiv(most, 64), p.count, 6), 64, 0, stream>>>(p);
+    launches++;
+    INCRMT_CKL("k_tail_pack");
+    return INCRMT_OK;
+}
+
+template <class T>
+int Multigrid::tail_launch() {
+    TailPlan<T> p;
+    int blocks, threads;
+    size_t smem;
+    const T *gi;
+    if constexpr (sizeof(T) == 8) gi = ginv;
+    else gi = ginvf;
+    if (!tail_plan<T>(lev, tail_level, px, py, gi, tail_max_blocks, p, blocks, threads, smem)) {
+        set_error("tail levels do not fit");
+        return INCRMT_ERR_CUDA;
+    }
+    if constexpr (sizeof(T) == 8) { p.z = lev[tail_level].z; p.b = lev[tail_level].b; }
+    else { p.z = lev[tail_level].zf; p.b = lev[tail_level].bf; }
+    cudaLaunchAttribute at[1];
+    cudaLaunchConfig_t c = tail_config(blocks, threads, smem, stream, at);
+    bool seq = false;
+    for (int k = 0; k < p.count; k++) seq = seq || p.lev[k].seq;
+    if (seq) INCRMT_CK(cudaLaunchKernelEx(&c, k_tail<T, true>, p));
+    else INCRMT_CK(cudaLaunchKernelEx(&c, k_tail<T, false>, p));
     launches++;
     INCRMT_CKL("k_tail");
     return INCRMT_OK;
 }
 
-int Multigrid::tail32() {
-    TailLevels<float> T{};
-    T.first = tail_level; T.count = static_cast<int>(lev.size()) - tail_level; T.px = px; T.py = py;
-    for (int k = 0; k < T.count; k++) {
-        const MgLevel &L = lev[tail_level + k];
-        T.m[k] = L.m; T.n[k] = L.n; T.N[k] = L.N; T.kx[k] = L.kx; T.ky[k] = L.ky;
-        T.z[k] = L.zf; T.b[k] = L.bf; T.st[k] = L.stf; T.P[k] = L.P;
-    }
-    T.ginv = ginvf;
-    const size_t sm = tail_layout(T, kTailSmemBudget);
-    k_tail<float><<<1, 1024, sm, stream>>>(T, kNu1, kNu2, kCoarseSweeps);
-    launches++;
-    INCRMT_CKL("k_tail");
-    return INCRMT_OK;
-}
+int Multigrid::tail64() { return tail_launch<double>(); }
+int Multigrid::tail32() { return tail_launch<float>(); }
 
 int Multigrid::norm2_rhs(const double *b, double *out_dev) {
     const long N = static_cast<long>(m) * n;

@@ -34,6 +34,8 @@ struct MgLevel {
     double *z2 = nullptr;  // second FP64 iterate buffer of the tile smoothers (all levels)
     double *P = nullptr;   // prolongation to the next level: four weights per unknown (all but the last)
     float *zf2 = nullptr;  // and the FP32 one
+    double *pk = nullptr;  // stencils and transfer weights packed for the tail kernel (its levels)
+    float *pkf = nullptr;
 };
 
 class Multigrid {
@@ -80,7 +82,9 @@ public:
     int lag_ld = 0;
     bool f32_stale = true;           // FP32 Galerkin stencils not cast since the last rebuild
     bool tiles = true;               // tile-fused smoothing where it applies
-    int tail_level = -1;             // first level run by the one-block tail kernel
+    int tail_level = -1;             // first level run by the tail kernel (mg_tail.cuh)
+    int tail_max_blocks = 1;         // blocks of its cluster at most
+    void *tail_pk = nullptr;         // its levels' packed stencils and weights
     cudaGraphExec_t gexec = nullptr; // captured V-cycle + norm
     cudaGraphExec_t setup_exec = nullptr;  // captured rebuild of the coarse levels
     long long setup_launches = 0;
@@ -163,6 +167,11 @@ private:
     int cast_levels();
     int cycle64(int l, const double *b0, double *z0);
     int cycle32(int l);
+    int choose_tail();
+    template <class T>
+    int tail_pack();
+    template <class T>
+    int tail_launch();
     int tail64();
     int vcycle_and_norm(int prec, const double *b, double *d_z, long N);
     int tail32();
