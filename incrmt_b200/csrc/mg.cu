@@ -3,6 +3,7 @@
 #include <cstring>
 #include <type_traits>
 #include "mg.cuh"
+#include "mg_stream.cuh"
 #include "mg_tail.cuh"
 
 namespace incrmt {
@@ -485,65 +486,6 @@ constexpr int gen_tile_smem() {
     return 11 * (TW + 8 * SWEEPS) * (TH + 8 * SWEEPS) * static_cast<int>(sizeof(T));
 }
 
-/** Tile-fused red-black Gauss-Seidel for a five-point operator (the fine MAC
- * system): the colours (0,0),(1,1) share no stencil edge, nor do (1,0),(0,1),
- * so the four-colour sweep is exactly two half-sweeps over (i+j) even, then
- * odd, with bitwise the same results. SWEEPS sweeps take 2*SWEEPS phases, so
- * the halo is 2*SWEEPS cells. Threads walk the tile as 32 x 8 (x fastest),
- * each row of a phase holding every second point. Reads zin, writes zout, and
- * handles periodic directions (even sizes) like k_smooth_tile. */
-template <class Op, class T, int SWEEPS, int TW, int TH>
-__global__ void __launch_bounds__(256) k_smooth_rb(Op op, const T *zin, T *zout, const T *b, int m, int n) {
-    constexpr int H = 2 * SWEEPS, LW = TW + 2 * H, LH = TH + 2 * H, NP = 2 * SWEEPS;
-    __shared__ T zs[LW * LH];
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int x0 = blockIdx.x * TW, y0 = blockIdx.y * TH;
-    const int gx0 = x0 - H, gy0 = y0 - H;
-    const bool px = op.px, py = op.py;
-    for (int lj = ty; lj < LH; lj += 8) {
-        int j = gy0 + lj;
-        if (py) j = wrap_index(j, n);
-        if (j < 0 || j >= n) continue;
-        for (int li = tx; li < LW; li += 32) {
-            int i = gx0 + li;
-            if (px) i = wrap_index(i, m);
-            if (i >= 0 && i < m) zs[li + LW * lj] = zin[i + static_cast<long>(m) * j];
-        }
-    }
-    __syncthreads();
-#pragma unroll 1
-    for (int p = 0; p < NP; p++) {
-        const int e = NP - 1 - p, parity = p & 1;
-        int ilo = x0 - e, ihi = x0 + TW - 1 + e, jlo = y0 - e, jhi = y0 + TH - 1 + e;
-        if (!px) {
-            if (ilo < 0) ilo = 0;
-            if (ihi > m - 1) ihi = m - 1;
-        }
-        if (!py) {
-            if (jlo < 0) jlo = 0;
-            if (jhi > n - 1) jhi = n - 1;
-        }
-        for (int j = jlo + ty; j <= jhi; j += 8) {
-            const int i0 = ilo + (((ilo + j) & 1) != parity);
-            const int jr = py ? wrap_index(j, n) : j;
-            for (int i = i0 + 2 * tx; i <= ihi; i += 64) {
-                const int lz = (i - gx0) + LW * (j - gy0);
-                const int ir = px ? wrap_index(i, m) : i;
-                zs[lz] = gs_update_s(op, ir, jr, zs, lz, LW, b[ir + static_cast<long>(m) * jr]);
-            }
-        }
-        __syncthreads();
-    }
-    for (int lj = H + ty; lj < H + TH; lj += 8) {
-        const int j = gy0 + lj;
-        if (j >= n) break;
-        for (int li = H + tx; li < H + TW; li += 32) {
-            const int i = gx0 + li;
-            if (i < m) zout[i + static_cast<long>(m) * j] = zs[li + LW * lj];
-        }
-    }
-}
-
 /** Coarse right-hand side b_c = P^T (b - A z), the fine residual formed on
  * the fly; also clears the coarse iterate. */
 template <class Op, class T>
@@ -1000,6 +942,18 @@ constexpr int kRedBlocks = 4 * kB200SMs;  // reduction grid: 4 x 148 blocks of 2
 inline dim3 grid2(int m, int n) { return dim3(cdiv(m, 32), cdiv(n, 8)); }
 const dim3 kBlk2(32, 8);
 
+/** Which systems' large levels run as a pipeline along y, and from how many
+ * unknowns on (mg_stream.cuh has both sides' times): the five-point one in
+ * both precisions, the FEM system in single. */
+template <class Op, class T>
+constexpr bool kStreams = false;
+template <class T>
+constexpr bool kStreams<MacOp<T>, T> = true;
+template <>
+constexpr bool kStreams<FemOp<float>, float> = true;
+template <class Op>
+constexpr long kStreamMin = Op::kFivePoint ? 512L * 512 : 1500L * 1500;
+
 /** The attributes a launch of k_tail needs. */
 template <class T, bool SEQ>
 cudaError_t set_tail_attr() {
@@ -1025,9 +979,10 @@ int smooth(Op op, T *z, T *zalt, const T *b, int m, int n, int sweeps, cudaStrea
         const dim3 b64(cdiv(m, 64), cdiv(n, 32)), b32(cdiv(m, 32), cdiv(n, 16)), b16(cdiv(m, 16), cdiv(n, 16));
         if (prof) { int r = prof->prof_begin(static_cast<double>(m) * n * 2 * bytes_per_unit); if (r) return r; }
         bool done = false;
-        if constexpr (Op::kFivePoint) {
-            if (static_cast<int>(b64.x * b64.y) >= 2 * kB200SMs) {
-                k_smooth_rb<Op, T, 2, 64, 32><<<b64, 256, 0, s>>>(op, z, zalt, b, m, n);
+        if constexpr (kStreams<Op, T>) {
+            if (static_cast<long>(m) * n >= kStreamMin<Op>) {
+                const StreamGrid<Op, T> sg(m, n);
+                k_smooth_stream<Op, T><<<sg.grid, 256, stream_elems<Op>() * sizeof(T), s>>>(op, z, zalt, b, m, n, sg.chunk);
                 done = true;
             }
         }
@@ -1193,6 +1148,9 @@ int Multigrid::build_hierarchy() {
         INCRMT_CK(cudaFuncSetAttribute(k_coarse_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(sizeof(double) * (2 * kDirectMax * kDirectMax + kDirectMax))));
     }
+    INCRMT_CK((set_stream_attr<MacOp<double>, double>()));
+    INCRMT_CK((set_stream_attr<MacOp<float>, float>()));
+    INCRMT_CK((set_stream_attr<FemOp<float>, float>()));
     INCRMT_CK((set_tail_attr<double, false>()));
     INCRMT_CK((set_tail_attr<double, true>()));
     INCRMT_CK((set_tail_attr<float, false>()));

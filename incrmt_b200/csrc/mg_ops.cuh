@@ -171,6 +171,11 @@ struct FemOp {
     __device__ __forceinline__ void coef9(int i, int j, T a[9]) const {
         T cdl, cdr, cul, cur;
         cells(i, j, cdl, cdr, cul, cur);
+        coef9_cells(i, j, cdl, cdr, cul, cur, a);
+    }
+
+    /** coef9 from the four cell values around the node (cells()). */
+    __device__ __forceinline__ void coef9_cells(int i, int j, T cdl, T cdr, T cul, T cur, T a[9]) const {
         const bool l = px || i > 0, r = px || i < m - 1, d = py || j > 0, u = py || j < n - 1;
         const bool fix = zpr && i == m - 1;
         a[4] = fm * (!d ? ((l ? cul : T(0)) + (r ? cur : T(0)))
@@ -217,9 +222,18 @@ struct FemOp {
     /** offdiag_s at a node on an edge of the grid (the cells from c). */
     template <bool CEN = false>
     __device__ __forceinline__ T offdiag_edge(int i, int j, const T *zs, int lz, int ldz, T &diag) const {
+        T cdl, cdr, cul, cur;
+        cells(i, j, cdl, cdr, cul, cur);
+        return offdiag_cells<CEN>(i, j, cdl, cdr, cul, cur, zs, lz, ldz, diag);
+    }
+
+    /** offdiag_edge, the four cell values around the node given. */
+    template <bool CEN = false>
+    __device__ __forceinline__ T offdiag_cells(int i, int j, T cdl, T cdr, T cul, T cur, const T *zs, int lz, int ldz,
+                                               T &diag) const {
         const T zc = CEN ? zs[lz] : T(0);
         T a[9];
-        coef9(i, j, a);
+        coef9_cells(i, j, cdl, cdr, cul, cur, a);
         diag = a[4];
         const bool l = px || i > 0, r = px || i < m - 1, d = py || j > 0, u = py || j < n - 1;
         T t = 0;

@@ -1,0 +1,54 @@
+"""The fine levels' pipelined smoothing (k_smooth_stream) against one launch per
+colour, bit for bit: grids just above its size threshold, odd sizes, strips
+whose last columns are one cell or a full strip, chunks of one row, and seams
+in either direction with densities that do not match across them."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # sys, m, n, x_prd, y_prd, zpr, mixed precision
+    (0, 512, 512, False, False, False, True),
+    (0, 513, 511, False, False, False, False),     # odd, just below and above in a direction
+    (0, 721, 601, False, False, True, True),       # 361 cells: a last strip of one cell
+    (0, 240, 1201, False, False, False, True),     # two full strips
+    (0, 16384, 17, False, False, False, False),    # more strips than blocks in a wave
+    (0, 17, 16384, False, False, False, False),    # one strip, many chunks
+    (0, 600, 512, True, True, False, False),
+    (0, 1536, 320, False, True, True, True),
+    (1, 1601, 1499, False, False, False, True),
+    (1, 1536, 1600, False, True, True, True),
+]
+
+
+@pytest.mark.parametrize("sys_,m,n,xp,yp,zpr,mixed", CASES)
+def test_stream_identical_to_colour_launches(gpu, sys_, m, n, xp, yp, zpr, mixed):
+    import torch
+    from incrmt_b200 import capi
+    s = capi.MGSolver(sys_, m, n, bx=-1 + 2 * m / max(m, n), by=-1 + 2 * n / max(m, n), x_prd=xp, y_prd=yp, zpr=zpr)
+    rng = np.random.default_rng(m * 7 + n)
+    rho = 1 + 2 * rng.random((n + 4, m + 4))
+    N = s.m_sys * s.n_sys
+    b = rng.standard_normal(N)
+    b -= b.mean()
+    z0 = rng.standard_normal(N)
+    bd = torch.tensor(b, device="cuda")
+    out = {}
+    for tiles in (True, False):
+        s.set_tiles(tiles)
+        s.set_density(rho)
+        z = torch.tensor(z0, device="cuda")
+        zm = torch.zeros(N, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        s.vcycle_device(bd.data_ptr(), z.data_ptr())
+        if mixed:  # one FP32 correction; the cap is its expected end
+            with pytest.raises(capi.IncrmtError) as e:
+                s.solve_device(bd.data_ptr(), zm.data_ptr(), max_vcycles=1, precision=capi.PREC_MIXED)
+            assert e.value.code == capi.ERR_NOCONV
+        torch.cuda.synchronize()
+        out[tiles] = (z.cpu().numpy(), zm.cpu().numpy())
+    assert np.isfinite(out[True][0]).all() and np.isfinite(out[True][1]).all()
+    assert np.array_equal(out[True][0], out[False][0])
+    assert np.array_equal(out[True][1], out[False][1])
+    s.close()
