@@ -275,261 +275,151 @@ __global__ void k_ls_copy_interface(LsGrid g, const LsObj *ob, const LsWin *win)
     if (o.s[ij] == 3 || o.s[ij] == 4) o.phi[ij] = o.phi_new[ij];
 }
 
-/** Marching direction: positive side (dir_positive) or negative side
- * (dir_negative), heap.hh:56-80. */
-template <bool POS>
-struct MarchDir {
-    __device__ static __forceinline__ bool cm(double a, double b) { return POS ? a < b : a > b; }
-    __device__ static __forceinline__ double ct(double a, double b) { return POS ? a + b : a - b; }
-};
-
-/** The second-order upwind stencil of the fast march for one point
- * (heap<d_option>::calc and helpers, heap.cc:177-376, 390-435), with the
- * "in" predicate supplied by the caller. */
-template <bool POS>
-struct March {
-    using D = MarchDir<POS>;
-    const LsGrid &g;
-    const double *phi;
-    const int *s0;        // status after the sign scan
-    const double *cur;    // current values of this side's candidates
-    double pv;            // current value of the point being evaluated
-    int lim_i, lim_j;
-    double dx, dy, dx2, dy2, dxbydy, dx2bydy2;
-
-    __device__ March(const LsGrid &g_, const double *phi_, const int *s0_, const double *cur_, double pv_)
-        : g(g_), phi(phi_), s0(s0_), cur(cur_), pv(pv_) {
-        dx = g.dx; dy = g.dy; dx2 = dx * dx; dy2 = dy * dy;
+/** Grid constants of the march's stencil. */
+struct MarchK {
+    double dx, dy, dx2, dxbydy, dx2bydy2;
+    // corner(h, v): index 2 h + v
+    double f2[4], i2[4], lim[4];
+    __device__ void set(const LsGrid &g) {
+        dx = g.dx; dy = g.dy;
+        dx2 = dx * dx;
+        const double dy2 = dy * dy;
         dxbydy = dx / dy; dx2bydy2 = dxbydy * dxbydy;
-    }
-    /** Value of a point as seen by the stencil: fixed points keep phi, this
-     * side's candidates their current value. */
-    __device__ __forceinline__ double val(int ij) const {
-        const int st = s0[ij];
-        return (POS ? st == 7 : st == 0) ? cur[ij] : phi[ij];
-    }
-    /** Whether a point counts as accepted before the one being evaluated:
-     * every point of the other side or of the interface, or a candidate of
-     * this side with a smaller current value. */
-    __device__ __forceinline__ bool in(int ij) const {
-        const int st = s0[ij];
-        if (POS ? st != 7 : st != 0) return true;
-        return D::cm(cur[ij], pv);
-    }
-    __device__ bool look(int ij, int o, bool ok2, double &e) const {
-        if (ok2 && in(ij + 2 * o)) {
-            const double f2 = val(ij + 2 * o), f1 = val(ij + o);
-            if (D::cm(f2, f1)) { e = 2 * f1 - 0.5 * f2; return true; }
-        }
-        e = val(ij + o);
-        return false;
-    }
-    __device__ double corner_bail(bool h, bool v, double a, double b) const {
-        const double ti = 2.0 / 3.0;
-        double ht = h ? D::ct(a, dx) * ti : D::ct(a, dx);
-        double vt = v ? D::ct(b, dy) * ti : D::ct(b, dy);
-        return D::cm(ht, vt) ? ht : vt;
-    }
-    __device__ double corner(bool h, bool v, double a, double b) const {
-        const double f2a = 2.25 * (dy2 + dx2), f2b = 2.25 * dy2 + dx2, f2c = dy2 + 2.25 * dx2, f2d = dy2 + dx2;
-        const double b1 = 2.25 * dx2 > dy2 ? 1 + 2.25 * dx2bydy2 : 1 + dy2 / (2.25 * dx2);
-        const double b2 = dx2 > dy2 ? 1 + dx2bydy2 : 1 + dy2 / dx2;
-        const double b3 = dx2 > 2.25 * dy2 ? 1 + dx2bydy2 / 2.25 : 1 + 2.25 * dy2 / dx2;
-        const double i2a = dy2 / f2a, i2b = dy2 / f2b, i2c = dy2 / f2c, i2d = dy2 / f2d;
-        double f;
-        if (h) {
-            if (v) {
-                f = 1.5 * (a - b); f *= f;
-                return f * b2 < f2a ? D::ct(a * 1.5 + b * 1.5 * dx2bydy2, dxbydy * sqrt(f2a - f)) * i2a
-                                    : corner_bail(true, true, a, b);
-            }
-            f = a - 1.5 * b; f *= f;
-            return f * b3 < f2b ? D::ct(a * 1.5 + b * dx2bydy2, dxbydy * sqrt(f2b - f)) * i2b
-                                : corner_bail(true, false, a, b);
-        }
-        if (v) {
-            f = 1.5 * a - b; f *= f;
-            return f * b1 < f2c ? D::ct(a + b * 1.5 * dx2bydy2, dxbydy * sqrt(f2c - f)) * i2c
-                                : corner_bail(false, true, a, b);
-        }
-        f = a - b; f *= f;
-        return f * b2 < f2d ? D::ct(a + b * dx2bydy2, dxbydy * sqrt(f2d - f)) * i2d
-                            : corner_bail(false, false, a, b);
-    }
-    __device__ double fourway(double a, double b, double c, double d) const {
-        double e = 2 * (c - a), f = 2 * (d - b), gg, h;
-        if (D::cm(e, f)) {
-            gg = e - a; h = e - b;
-            if (D::cm(gg, 0)) gg = 0;
-            if (D::cm(h, 0)) h = 0;
-            if (gg * gg + h * h * dx2bydy2 < dx2) {
-                gg = 1.5 * f - c; h = f - b;
-                if (D::cm(gg, 0)) gg = 0;
-                if (D::cm(h, 0)) h = 0;
-                if (gg * gg + h * h * dx2bydy2 < dx2) return corner(true, true, c, d);
-                return corner(true, false, c, b);
-            }
-            return corner(false, false, a, b);
-        }
-        gg = f - a; h = f - b;
-        if (D::cm(gg, 0)) gg = 0;
-        if (D::cm(h, 0)) h = 0;
-        if (gg * gg + h * h * dx2bydy2 < dx2) {
-            gg = e - a; h = 1.5 * e - d;
-            if (D::cm(gg, 0)) gg = 0;
-            if (D::cm(h, 0)) h = 0;
-            if (gg * gg + h * h * dx2bydy2 < dx2) return corner(true, true, c, d);
-            return corner(false, true, a, d);
-        }
-        return corner(false, false, a, b);
-    }
-    __device__ double threeway1(bool h1, bool h2, bool v, double a, double c, double b) const {
-        double d;
-        if (h1) {
-            if (h2) { d = D::cm(a, c) ? a : c; return corner(true, v, d, b); }
-            d = 2 * (a - c);
-            double e = d - c, f = (v ? 1.5 * d : d) - b;
-            if (D::cm(e, 0)) e = 0;
-            if (D::cm(f, 0)) f = 0;
-            return e * e + f * f * dx2bydy2 < dx2 ? corner(true, v, a, b) : corner(false, v, c, b);
-        }
-        if (h2) {
-            d = 2 * (c - a);
-            double e = d - a, f = (v ? 1.5 * d : d) - b;
-            if (D::cm(e, 0)) e = 0;
-            if (D::cm(f, 0)) f = 0;
-            return e * e + f * f * dx2bydy2 < dx2 ? corner(true, v, c, b) : corner(false, v, a, b);
-        }
-        d = D::cm(a, c) ? a : c;
-        return corner(false, v, d, b);
-    }
-    __device__ double threeway2(bool h, bool v1, bool v2, double b, double a, double c) const {
-        double d;
-        if (v1) {
-            if (v2) { d = D::cm(a, c) ? a : c; return corner(h, true, b, d); }
-            d = 2 * (a - c);
-            double e = d - c, f = (h ? 1.5 * d : d) - b;
-            if (D::cm(e, 0)) e = 0;
-            if (D::cm(f, 0)) f = 0;
-            return f * f + e * e * dx2bydy2 < dx2 ? corner(h, true, b, a) : corner(h, false, b, c);
-        }
-        if (v2) {
-            d = 2 * (c - a);
-            double e = d - a, f = (h ? 1.5 * d : d) - b;
-            if (D::cm(e, 0)) e = 0;
-            if (D::cm(f, 0)) f = 0;
-            return f * f + e * e * dx2bydy2 < dx2 ? corner(h, true, b, c) : corner(h, false, b, a);
-        }
-        d = D::cm(a, c) ? a : c;
-        return corner(h, false, b, d);
-    }
-    /** heap::calc (heap.cc:177-263) at point (i,j). */
-    __device__ double calc(int i, int j) const {
-        const int P = g.P, ij = j * P + i, m = g.mL, n = g.nL;
-        const int L = -1, R = 1, Dn = -P, U = P;
-        double a, b, c, d;
-        const double ti = 2.0 / 3.0;
-        auto look_l = [&](double &e) { return look(ij, L, i > 1, e); };
-        auto look_r = [&](double &e) { return look(ij, R, i < m - 2, e); };
-        auto look_d = [&](double &e) { return look(ij, Dn, j > 1, e); };
-        auto look_u = [&](double &e) { return look(ij, U, j < n - 2, e); };
-        if (j > 0 && in(ij - P)) {
-            if (j < n - 1 && in(ij + P)) {
-                if (i < m - 1 && in(ij + 1)) {
-                    if (i > 0 && in(ij - 1)) {
-                        if (look_d(a)) {
-                            if (look_u(c)) {
-                                d = D::cm(a, c) ? a : c;
-                                bool hl = look_l(a), hr = look_r(c);
-                                return threeway1(hl, hr, true, a, c, d);
-                            } else {
-                                if (look_l(b)) {
-                                    if (look_r(d)) { b = D::cm(b, d) ? b : d; return threeway2(true, true, false, b, a, c); }
-                                    return fourway(d, c, b, a);
-                                } else {
-                                    if (look_r(d)) return fourway(b, c, d, a);
-                                    b = D::cm(b, d) ? b : d;
-                                    return threeway2(false, true, false, b, a, c);
-                                }
-                            }
-                        } else {
-                            if (look_u(c)) {
-                                if (look_l(b)) {
-                                    if (look_r(d)) { b = D::cm(b, d) ? b : d; return threeway2(true, true, false, b, c, a); }
-                                    return fourway(d, a, b, c);
-                                } else {
-                                    if (look_r(d)) return fourway(b, a, d, c);
-                                    b = D::cm(b, d) ? b : d;
-                                    return threeway2(false, true, false, b, c, a);
-                                }
-                            } else {
-                                d = D::cm(a, c) ? a : c;
-                                bool hl = look_l(a), hr = look_r(c);
-                                return threeway1(hl, hr, false, a, c, d);
-                            }
-                        }
-                    } else {
-                        bool h = look_r(b), v1 = look_u(a), v2 = look_d(c);
-                        return threeway2(h, v1, v2, b, a, c);
-                    }
-                } else {
-                    if (i > 0 && in(ij - 1)) {
-                        bool h = look_l(b), v1 = look_u(a), v2 = look_d(c);
-                        return threeway2(h, v1, v2, b, a, c);
-                    }
-                    c = look_d(a) ? D::ct(a, dy) * ti : D::ct(a, dy);
-                    d = look_u(b) ? D::ct(b, dy) * ti : D::ct(b, dy);
-                    return D::cm(c, d) ? c : d;
-                }
-            } else {
-                if (i < m - 1 && in(ij + 1)) {
-                    if (i > 0 && in(ij - 1)) {
-                        bool hl = look_l(a), hr = look_r(c), v = look_d(b);
-                        return threeway1(hl, hr, v, a, c, b);
-                    }
-                    bool h = look_r(a), v = look_d(b);
-                    return corner(h, v, a, b);
-                } else {
-                    if (i > 0 && in(ij - 1)) { bool h = look_l(a), v = look_d(b); return corner(h, v, a, b); }
-                    return look_d(a) ? D::ct(a, dy) * ti : D::ct(a, dy);
-                }
-            }
-        } else {
-            if (j < n - 1 && in(ij + P)) {
-                if (i < m - 1 && in(ij + 1)) {
-                    if (i > 0 && in(ij - 1)) {
-                        bool hl = look_l(a), hr = look_r(c), v = look_u(b);
-                        return threeway1(hl, hr, v, a, c, b);
-                    }
-                    bool h = look_r(a), v = look_u(b);
-                    return corner(h, v, a, b);
-                } else {
-                    if (i > 0 && in(ij - 1)) { bool h = look_l(a), v = look_u(b); return corner(h, v, a, b); }
-                    return look_u(a) ? D::ct(a, dy) * ti : D::ct(a, dy);
-                }
-            } else {
-                if (i < m - 1 && in(ij + 1)) {
-                    if (i > 0 && in(ij - 1)) {
-                        c = look_l(a) ? D::ct(a, dx) * ti : D::ct(a, dx);
-                        d = look_r(b) ? D::ct(b, dx) * ti : D::ct(b, dx);
-                        return D::cm(c, d) ? c : d;
-                    }
-                    return look_r(a) ? D::ct(a, dx) * ti : D::ct(a, dx);
-                } else {
-                    if (i > 0 && in(ij - 1)) return look_l(a) ? D::ct(a, dx) * ti : D::ct(a, dx);
-                    return 0;
-                }
-            }
-        }
+        f2[3] = 2.25 * (dy2 + dx2); f2[2] = 2.25 * dy2 + dx2; f2[1] = dy2 + 2.25 * dx2; f2[0] = dy2 + dx2;
+        lim[1] = 2.25 * dx2 > dy2 ? 1 + 2.25 * dx2bydy2 : 1 + dy2 / (2.25 * dx2);
+        lim[3] = lim[0] = dx2 > dy2 ? 1 + dx2bydy2 : 1 + dy2 / dx2;
+        lim[2] = dx2 > 2.25 * dy2 ? 1 + dx2bydy2 / 2.25 : 1 + 2.25 * dy2 / dx2;
+        for (int k = 0; k < 4; k++) i2[k] = dy2 / f2[k];
     }
 };
 
-/** Whether a point has at least one 4-neighbour that counts as "in". */
-template <bool POS>
-__device__ __forceinline__ bool any_in(const March<POS> &mr, int i, int j) {
-    const int P = mr.g.P, ij = j * P + i;
-    return (i > 0 && mr.in(ij - 1)) || (i < mr.g.mL - 1 && mr.in(ij + 1)) ||
-           (j > 0 && mr.in(ij - P)) || (j < mr.g.nL - 1 && mr.in(ij + P));
+/** The second-order upwind stencil of the fast march (heap<d_option>::calc and
+ * its helpers, heap.cc:177-376, 390-435) for one candidate, staged at q of
+ * arrays with row pitch P: ph the level set, st the status after the sign
+ * scan, cur the candidates' values. A point counts as accepted ("in") if it
+ * is not a candidate of this side (whose far status is `far`), or one with a
+ * smaller value. The negative side is the positive one with every value
+ * negated (sg = -1, exact), so one copy of the code serves both. The case
+ * analysis only selects which two neighbour values, with which orders, enter
+ * the final quadratic (h, v: second order along x, y; a, b: the values).
+ * Returns the point's own value if no neighbour is in. */
+__device__ __forceinline__ double march_value(const MarchK &K, int P, const double *ph, const unsigned char *st,
+                                              const double *cur, int q, int far, double sg, double own, bool l1, bool l2,
+                                              bool r1, bool r2, bool d1, bool d2, bool u1, bool u2) {
+    const double pv = sg * own;
+    auto val = [&](int k) { return sg * (st[k] == far ? cur[k] : ph[k]); };
+    auto in = [&](int k) { return st[k] != far || sg * cur[k] < pv; };
+    // The neighbour at offset o: whether it is in, its value, extrapolated to
+    // second order where the next one is in and smaller (second).
+    auto look = [&](int o, bool one, bool two, double &e, bool &second) {
+        second = false;
+        e = 0;
+        if (!one || !in(q + o)) return false;
+        e = val(q + o);
+        if (two && in(q + 2 * o)) {
+            const double f2 = val(q + 2 * o);
+            if (f2 < e) {
+                e = 2 * e - 0.5 * f2;
+                second = true;
+            }
+        }
+        return true;
+    };
+    double xl, xr, yd, yu;
+    bool hl, hr, vd, vu;
+    const bool L = look(-1, l1, l2, xl, hl), R = look(1, r1, r2, xr, hr);
+    const bool D = look(-P, d1, d2, yd, vd), U = look(P, u1, u2, yu, vu);
+    const double ti = 2.0 / 3.0;
+    if (!L && !R && !D && !U) return own;
+    if (!D && !U) {
+        const double c = hl ? (xl + K.dx) * ti : xl + K.dx, d = hr ? (xr + K.dx) * ti : xr + K.dx;
+        return sg * (L && R ? (c < d ? c : d) : (L ? c : d));
+    }
+    if (!L && !R) {
+        const double c = vd ? (yd + K.dy) * ti : yd + K.dy, d = vu ? (yu + K.dy) * ti : yu + K.dy;
+        return sg * (D && U ? (c < d ? c : d) : (D ? c : d));
+    }
+    // Differences below zero count as zero in the tests that follow.
+    auto near = [&](double e, double f) {
+        if (e < 0) e = 0;
+        if (f < 0) f = 0;
+        return e * e + f * f * K.dx2bydy2 < K.dx2;
+    };
+    bool h, v;
+    double a, b;
+    // Both x neighbours of first and second order n, s (threeway1), or both y
+    // ones (threeway2): the second-order one where it is near.
+    auto three_x = [&](double n, double s, bool vv, double y) {
+        const double d = 2 * (s - n);
+        h = near(d - n, (vv ? 1.5 * d : d) - y);
+        v = vv;
+        a = h ? s : n;
+        b = y;
+    };
+    auto three_y = [&](double n, double s, bool hh, double x) {
+        const double d = 2 * (s - n);
+        v = near((hh ? 1.5 * d : d) - x, d - n);
+        h = hh;
+        a = x;
+        b = v ? s : n;
+    };
+    if (L && R && D && U && vd != vu) {
+        const double ys = vd ? yd : yu, yn = vd ? yu : yd;
+        if (hl == hr) {
+            three_y(yn, ys, hl, xl < xr ? xl : xr);
+        } else {
+            // fourway: first and second order along both axes
+            const double xs = hl ? xl : xr, xn = hl ? xr : xl;
+            const double e = 2 * (xs - xn), f = 2 * (ys - yn);
+            if (e < f) {
+                h = near(e - xn, e - yn);
+                v = h && near(1.5 * f - xs, f - yn);
+            } else {
+                v = near(f - xn, f - yn);
+                h = v && near(e - xn, 1.5 * e - ys);
+            }
+            a = h ? xs : xn;
+            b = v ? ys : yn;
+        }
+    } else if (L && R) {
+        const double y = D && U ? (yd < yu ? yd : yu) : (D ? yd : yu);
+        const bool vv = D ? vd : vu;
+        if (hl != hr) {
+            three_x(hl ? xr : xl, hl ? xl : xr, vv, y);
+        } else {
+            h = hl; v = vv;
+            a = xl < xr ? xl : xr;
+            b = y;
+        }
+    } else if (D && U) {
+        const double x = L ? xl : xr;
+        const bool hh = L ? hl : hr;
+        if (vd != vu) {
+            three_y(vd ? yu : yd, vd ? yd : yu, hh, x);
+        } else {
+            h = hh; v = vd;
+            a = x;
+            b = yd < yu ? yd : yu;
+        }
+    } else {
+        h = L ? hl : hr; v = D ? vd : vu;
+        a = L ? xl : xr;
+        b = D ? yd : yu;
+    }
+    const int k = 2 * h + v;
+    double f0 = h == v ? a - b : (h ? __fma_rn(-1.5, b, a) : __fma_rn(1.5, a, -b));
+    if (h && v) f0 = __dmul_rn(1.5, f0);
+    const double f = __dmul_rn(f0, f0);
+    if (__dmul_rn(f, K.lim[k]) < K.f2[k]) {
+        // (roundings written out: a shape aligned with the grid has many equal
+        // values, whose order decides which of them others see)
+        const double bv = v ? b * 1.5 : b;
+        const double e = h ? __fma_rn(a, 1.5, __dmul_rn(bv, K.dx2bydy2)) : __fma_rn(bv, K.dx2bydy2, a);
+        return sg * __dmul_rn(__fma_rn(K.dxbydy, sqrt(__dsub_rn(K.f2[k], f)), e), K.i2[k]);
+    }
+    // the two directions apart (corner_bail)
+    const double ht = h ? (a + K.dx) * ti : a + K.dx, vt = v ? (b + K.dy) * ti : b + K.dy;
+    return sg * (ht < vt ? ht : vt);
 }
 
 constexpr double kUnset = 1e300;
@@ -551,11 +441,10 @@ __global__ void k_ls_fim_init(LsGrid g, const LsObj *ob, const LsWin *win) {
 /** Final values and clean-up (heap::march acceptance, levelset::clean,
  * levelset.cc:408-413): far points whose value fell inside the band limit are
  * accepted (5 / 2); every point outside the band is set to the band limit. */
-__global__ void k_ls_finish(LsGrid g, const LsObj *ob, const LsWin *win) {
+__global__ void k_ls_finish(LsGrid g, const LsObj *ob, const LsWin *win, bool in_b) {
     int i, j;
     if (!ls_point(g, win, i, j)) return;
-    // After the last (unchanging) sweep both buffers hold the final values.
-    const double *cur = ob[blockIdx.z].a;
+    const double *cur = in_b ? ob[blockIdx.z].b : ob[blockIdx.z].a;
     int *s = ob[blockIdx.z].s;
     double *phi = ob[blockIdx.z].phi;
     const int ij = j * g.P + i, st = s[ij];
@@ -762,100 +651,215 @@ __global__ void k_ls_dilate(LsGrid g, const LsObj *ob, const LsWin *win, int R) 
     out[j * g.P + i] = v;
 }
 
-/** Lists the far points (status 0 or 7) inside the dilated interface region:
- * the only points the march can reach within the band limit. */
-__global__ void k_ls_collect_candidates(LsGrid g, const LsObj *ob, const LsWin *win, int *list, int *list_k, int *count, int cap,
-                                        int *overflow) {
-    int i, j;
-    if (!ls_point(g, win, i, j)) return;
-    const LsObj &o = ob[blockIdx.z];
-    const int ij = j * g.P + i, st = o.s[ij];
-    if ((st == 0 || st == 7) && o.ia[ij]) ls_list_push(list, list_k, count, cap, overflow, ij, blockIdx.z);
+/** Whether a point is a candidate of the march: a far point (status 0 or 7)
+ * inside the dilated interface region (ia), the only points the march can
+ * reach within the band limit. */
+__device__ __forceinline__ bool ls_candidate(const LsObj &o, int ij) {
+    const int st = o.s[ij];
+    return (st == 0 || st == 7) && o.ia[ij];
+}
+
+/** Lists the tiles (TILE x TILE points of an object's window) that hold
+ * candidates as (x | y << 16, object), one block of 256 threads per tile. */
+template <int TILE>
+__global__ void k_ls_collect_tiles(LsGrid g, const LsObj *ob, const LsWin *win, int *list, int *list_k, int *count, int cap,
+                                   int *overflow) {
+    const LsWin w = win[blockIdx.z];
+    const int xe = min(w.x1, g.mL), ye = min(w.y1, g.nL);
+    bool any = false;
+    for (int t = threadIdx.x; t < TILE * TILE; t += blockDim.x) {
+        const int i = w.x0 + blockIdx.x * TILE + t % TILE, j = w.y0 + blockIdx.y * TILE + t / TILE;
+        if (i < xe && j < ye && ls_candidate(ob[blockIdx.z], j * g.P + i)) any = true;
+    }
+    if (__syncthreads_or(any) && threadIdx.x == 0)
+        ls_list_push(list, list_k, count, cap, overflow, blockIdx.x | blockIdx.y << 16, blockIdx.z);
 }
 
 /** Threads per block of the cooperative sweeps: one block per SM (the grid
- * barrier costs more with more blocks), as many threads as the registers
- * allow, so that a candidate list of ~1e5 points takes about one pass per
- * sweep and each SM has many warps to hide the stencil's dependent loads. */
+ * barrier costs more with more blocks). */
 constexpr int kFimThreads = 1024;
 constexpr int kExtrapThreads = 512;
 
-/** Whether any point the stencil of (i,j) reads (up to two cells along
- * each axis) changed in the previous sweep. */
-__device__ __forceinline__ bool stencil_changed(const LsGrid &g, const unsigned char *chg, int i, int j) {
-    const int P = g.P, ij = j * P + i;
-    if (chg[ij]) return true;
-    for (int d = 1; d <= 2; d++) {
-        if (i - d >= 0 && chg[ij - d]) return true;
-        if (i + d < g.mL && chg[ij + d]) return true;
-        if (j - d >= 0 && chg[ij - d * P]) return true;
-        if (j + d < g.nL && chg[ij + d * P]) return true;
-    }
-    return false;
+/** The march's staging: tiles of TILE x TILE points, SWEEPS sweeps between grid
+ * barriers, the halo they need (the stencil and its change marks reach two
+ * points), and the staged region. */
+template <int TILE, int SWEEPS>
+struct Fim {
+    static constexpr int kHalo = 2 * SWEEPS, kReg = TILE + 2 * kHalo, kPoints = kReg * kReg, kRound = (kPoints + 31) & ~31;
+    static constexpr size_t kSmem = kPoints * (3 * sizeof(double) + 2 * sizeof(short) + 3);
+};
+
+/** Appends q to a shared-memory list for the lanes that ask for it (all lanes
+ * of the warp call). */
+__device__ __forceinline__ void fim_push(bool on, int q, unsigned short *list, int *n) {
+    const unsigned votes = __ballot_sync(0xffffffffu, on);
+    if (!votes) return;
+    int base = 0;
+    if ((threadIdx.x & 31) == 0) base = atomicAdd(n, __popc(votes));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (on) list[base + __popc(votes & ((1u << (threadIdx.x & 31)) - 1))] = static_cast<unsigned short>(q);
 }
 
 /** All sweeps of the march fixed point in one cooperative launch: every
- * sweep evaluates the stencil at the listed candidates (Jacobi, reading cur,
- * writing nxt), a grid barrier follows, and the loop ends after the first
- * sweep that changed nothing. A candidate whose stencil inputs did not change
- * in the previous sweep keeps its value (its stencil would return it again),
- * so later sweeps only touch the moving front; each object's ca/cb are
- * per-point change marks of the previous and the current sweep (cleared by
- * k_ls_fim_init) and a/b its values, swapped every sweep. The list holds the
- * candidates of every object, so all bands settle in the same launch.
- * flags[0..2] rotate as per-sweep change flags; flags[3] receives the number
- * of sweeps and flags[4] 1 if converged. */
-__global__ void __launch_bounds__(kFimThreads, 1) k_ls_fim_coop(LsGrid g, const LsObj *ob, const int *list, const int *list_k, const int *countp,
-                              int cap, int *flags, int max_sweeps) {
+ * sweep evaluates the stencil at the candidates (Jacobi, reading cur, writing
+ * nxt) and the loop ends after the first sweep that changed nothing. A
+ * candidate whose stencil inputs did not change in the previous sweep keeps
+ * its value (its stencil would return it again), so later sweeps only touch
+ * the moving front.
+ *
+ * The blocks take the listed tiles (of every object), stage each with its
+ * halo in shared memory and run SWEEPS sweeps there, the halo's points
+ * redundantly in every tile that holds them, the region one sweep is valid in
+ * shrinking by the stencil's reach; a grid barrier then exchanges the tiles
+ * through global memory. The values are those of one barrier per sweep: a
+ * sweep costs its evaluations, gathered into full warps and reading shared
+ * memory, instead of some six round trips to L2 and a barrier, and the sweeps
+ * past the last one of a batch change nothing (no marks are left). o.a/o.b
+ * hold the values and o.ca/o.cb the change marks, swapped every batch;
+ * k_ls_fim_init sets them where no tile is listed.
+ *
+ * It is bound by the evaluations of the busiest SM (some 600 instructions per
+ * warp, half of them FP64) and their latency: about 2-4 us per sweep against
+ * 10 us of a sweep over global memory with a barrier each. Measured (B200, us
+ * per call before -> now): rotor 128^2 336 -> 108, 1024^2 457 -> 163; 32 bodies
+ * 1024 x 2048 503 -> 395; flag 2048^2 892 -> 316. Lists built by the points that
+ * change, instead of the marks' scan, took 185 us where this takes 149.
+ *
+ * flags[0..2] rotate as per-batch masks of the sweeps that changed something;
+ * flags[3] receives the number of sweeps and flags[4] 1 if converged; after
+ * ceil(sweeps / SWEEPS) batches the values are in o.b if that is odd. */
+template <int TILE, int SWEEPS>
+__global__ void __launch_bounds__(kFimThreads, 1) k_ls_fim_coop(LsGrid g, const LsObj *ob, const LsWin *win, const int *list,
+                              const int *list_k, const int *countp, int cap, int *flags, int max_sweeps) {
     namespace cg = cooperative_groups;
     cg::grid_group grid = cg::this_grid();
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
-    const int count = min(*countp, cap);
-    int it = 0;
+    using F = Fim<TILE, SWEEPS>;
+    constexpr int REG = F::kReg, RR = F::kPoints;
+    extern __shared__ __align__(16) double fim_smem[];
+    double *va = fim_smem, *vb = va + RR, *ph = vb + RR;
+    unsigned short *cand = reinterpret_cast<unsigned short *>(ph + RR), *work = cand + RR;
+    unsigned char *st = reinterpret_cast<unsigned char *>(work + RR), *ma = st + RR, *mb = ma + RR;
+    __shared__ int ncand, nwork;
+    __shared__ MarchK mk;
+    const int tid = threadIdx.x, count = min(*countp, cap);
+    if (tid == 0) mk.set(g);
     bool done = false;
-    for (; it < max_sweeps; it++) {
-        if (tid == 0) flags[(it + 1) % 3] = 0;
-        const bool odd = it & 1;
-        // Where the second-order stencil is not monotone, the plain sweeps can
-        // cycle between two states instead of settling (seen on thin solids at
-        // fine grids). After half the sweep budget each value may then only
-        // move towards the interface, which settles; flags[12] records it.
-        const bool monotone = it >= max_sweeps / 2;
-        if (monotone && tid == 0) flags[12] = 1;
-        bool ch = false;
-        for (int t = tid; t < count; t += nth) {
-            const LsObj &o = ob[list_k[t]];
-            const double *cur = odd ? o.b : o.a;
-            double *nxt = odd ? o.a : o.b;
-            const unsigned char *cprev = odd ? o.cb : o.ca;
-            unsigned char *cnow = odd ? o.ca : o.cb;
-            const int ij = list[t], i = ij % g.P, j = ij / g.P, st = o.s[ij];
-            const double old = cur[ij];
-            double v = old;
-            if (it == 0 || stencil_changed(g, cprev, i, j)) {
-                if (st == 7) {
-                    March<true> mr(g, o.phi, o.s, cur, old);
-                    if (any_in(mr, i, j)) v = mr.calc(i, j);
-                    if (monotone && v > old) v = old;
-                } else {
-                    March<false> mr(g, o.phi, o.s, cur, old);
-                    if (any_in(mr, i, j)) v = mr.calc(i, j);
-                    if (monotone && v < old) v = old;
+    int it0 = 0;
+    for (int batch = 0; it0 < max_sweeps; batch++, it0 += SWEEPS) {
+        if (blockIdx.x == 0 && tid == 0) flags[(batch + 1) % 3] = 0;
+        const bool odd = batch & 1;
+        for (int tile = blockIdx.x; tile < count; tile += gridDim.x) {
+            const LsObj &o = ob[list_k[tile]];
+            const LsWin w = win[list_k[tile]];
+            const double *gin = odd ? o.b : o.a;
+            double *gout = odd ? o.a : o.b;
+            const unsigned char *cin = odd ? o.cb : o.ca;
+            unsigned char *cout = odd ? o.ca : o.cb;
+            const int x0 = w.x0 + (list[tile] & 0xffff) * TILE - F::kHalo;
+            const int y0 = w.y0 + (list[tile] >> 16) * TILE - F::kHalo;
+            const int xe = min(w.x1, g.mL), ye = min(w.y1, g.nL);
+            __syncthreads();  // the tile before is written out
+            if (tid == 0) ncand = 0;
+            __syncthreads();
+            for (int t = tid; t < F::kRound; t += kFimThreads) {
+                const int i = x0 + t % REG, j = y0 + t / REG;
+                double v = 0, p = 0;
+                unsigned char s = 4, mark = 0;
+                bool c = false;
+                // Outside the window nothing is a candidate, and no stencil
+                // of one reaches there.
+                if (t < RR && i >= w.x0 && i < xe && j >= w.y0 && j < ye) {
+                    const int ij = j * g.P + i;
+                    s = static_cast<unsigned char>(o.s[ij]);
+                    p = o.phi[ij];
+                    v = gin[ij];
+                    mark = cin[ij];
+                    c = (s == 0 || s == 7) && o.ia[ij];
+                }
+                if (t < RR) {
+                    va[t] = vb[t] = v;
+                    ph[t] = p;
+                    st[t] = s;
+                    ma[t] = mark;
+                    mb[t] = 0;
+                }
+                fim_push(c, t, cand, &ncand);
+            }
+            __syncthreads();
+            const int nc = ncand;
+            int mask = 0;
+#pragma unroll 1
+            for (int k = 0; k < SWEEPS; k++) {
+                const int it = it0 + k, ring = 2 * (k + 1), span = REG - 2 * ring;
+                // Where the second-order stencil is not monotone, the plain sweeps can
+                // cycle between two states instead of settling (seen on thin solids at
+                // fine grids). After half the sweep budget each value may then only
+                // move towards the interface, which settles; flags[12] records it.
+                const bool monotone = it >= max_sweeps / 2;
+                const double *cur = k & 1 ? vb : va;
+                double *nxt = k & 1 ? va : vb;
+                const unsigned char *cprev = k & 1 ? mb : ma;
+                unsigned char *cnow = k & 1 ? ma : mb;
+                // The candidates that keep their values are copied; the others
+                // are listed, so that full warps evaluate them.
+                if (tid == 0) nwork = 0;
+                __syncthreads();
+                for (int t = tid; t < ((nc + 31) & ~31); t += kFimThreads) {
+                    const int q = t < nc ? cand[t] : 0, lx = q % REG - ring, ly = q / REG - ring;
+                    bool eval = false;
+                    if (t < nc && lx >= 0 && lx < span && ly >= 0 && ly < span) {
+                        const unsigned char *m0 = cprev + q;
+                        eval = it == 0 || (m0[0] | m0[-1] | m0[1] | m0[-2] | m0[2] | m0[-REG] | m0[REG] | m0[-2 * REG] |
+                                           m0[2 * REG]);
+                        if (!eval) {
+                            nxt[q] = cur[q];
+                            cnow[q] = 0;
+                        }
+                    }
+                    fim_push(eval, q, work, &nwork);
+                }
+                __syncthreads();
+                const int nw = nwork;
+                bool ch = false;
+                for (int t = tid; t < nw; t += kFimThreads) {
+                    const int q = work[t], lx = q % REG, ly = q / REG, i = x0 + lx, j = y0 + ly;
+                    const double old = cur[q], sg = st[q] == 7 ? 1.0 : -1.0;
+                    double v = march_value(mk, REG, ph, st, cur, q, st[q], sg, old, i > 0, i > 1, i < g.mL - 1, i < g.mL - 2,
+                                           j > 0, j > 1, j < g.nL - 1, j < g.nL - 2);
+                    if (monotone && sg * v > sg * old) v = old;
+                    nxt[q] = v;
+                    // Changes in the last bits (the tail of the fixed point) do not
+                    // count: the sweeps end once every value is settled to 1e-13.
+                    const bool c = fabs(v - old) > 1e-13 * fabs(v);
+                    cnow[q] = c;
+                    if (c && lx >= F::kHalo && lx < F::kHalo + TILE && ly >= F::kHalo && ly < F::kHalo + TILE) ch = true;
+                }
+                if (__syncthreads_or(ch)) mask |= 1 << k;
+            }
+            if (mask && tid == 0) atomicOr(&flags[batch % 3], mask);
+            for (int t = tid; t < TILE * TILE; t += kFimThreads) {
+                const int lx = F::kHalo + t % TILE, ly = F::kHalo + t / TILE, q = ly * REG + lx;
+                const int i = x0 + lx, j = y0 + ly;
+                if (i < xe && j < ye) {
+                    gout[j * g.P + i] = SWEEPS & 1 ? vb[q] : va[q];
+                    cout[j * g.P + i] = SWEEPS & 1 ? mb[q] : ma[q];
                 }
             }
-            nxt[ij] = v;
-            // Changes in the last bits (the tail of the fixed point) do not
-            // count: the sweeps end once every value is settled to 1e-13.
-            const bool c = fabs(v - old) > 1e-13 * fabs(v);
-            cnow[ij] = c;
-            if (c) ch = true;
         }
-        if (__syncthreads_or(ch) && threadIdx.x == 0) flags[it % 3] = 1;
         grid.sync();
-        const int c = *reinterpret_cast<volatile int *>(&flags[it % 3]);
-        if (!c) { done = true; break; }
+        const int mask = *reinterpret_cast<volatile int *>(&flags[batch % 3]);
+        const int last = __ffs(~mask) - 1;  // the first sweep that changed nothing
+        if (last < SWEEPS && it0 + last < max_sweeps) {
+            it0 += last + 1;
+            done = true;
+            break;
+        }
     }
-    if (tid == 0) { flags[3] = done ? it + 1 : it; flags[4] = done ? 1 : 0; }
+    if (blockIdx.x == 0 && tid == 0) {
+        flags[3] = done ? it0 : max_sweeps;
+        flags[4] = done ? 1 : 0;
+        flags[12] = flags[3] > max_sweeps / 2 ? 1 : 0;
+    }
 }
 
 /** All sweeps of the extrapolation wavefront in one cooperative launch (same

@@ -22,6 +22,12 @@ namespace incrmt {
 namespace {
 const dim3 kB2(32, 8);
 inline dim3 g2(int m, int n) { return dim3(cdiv(m, 32), cdiv(n, 8)); }
+/** Sweeps per grid barrier of the march (k_ls_fim_coop), and its tile sizes:
+ * the small one where its tiles, one per SM, take one round (a sweep then costs
+ * what one SM needs for a tile), else the large one, whose halo is the smaller
+ * share. Measured (B200, us per call, 16 against 32 wide): rotor 128^2 108 /
+ * 149, 1024^2 283 / 163; 32 bodies 1024 x 2048 594 / 395; flag 2048^2 379 / 316. */
+constexpr int kFimSweeps = 4, kFimSmall = 16, kFimLarge = 32;
 constexpr int kLsMaxSweeps = 400;       // cap of the fixed-point sweeps of one march
 constexpr int kExtrapMaxSweeps = 1000;  // cap of the extrapolation wavefront sweeps
 constexpr int kLearnedStrikes = 8;      // rejected learned guesses in a row ...
@@ -300,8 +306,13 @@ int Sim::create(const incrmt_grid *gr, const incrmt_phys *ph) {
         INCRMT_CK(cudaGetDevice(&dev));
         INCRMT_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         // One block per SM: the grid barrier of the cooperative sweeps costs
-        // more with more blocks, and the candidate lists are ~1e4-1e5 points.
-        INCRMT_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_ls_fim_coop, kFimThreads, 0));
+        // more with more blocks.
+        const auto fim = k_ls_fim_coop<kFimLarge, kFimSweeps>;  // (the small tiles need less shared memory)
+        constexpr size_t fsm = Fim<kFimLarge, kFimSweeps>::kSmem;
+        INCRMT_CK(cudaFuncSetAttribute(fim, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(fsm)));
+        INCRMT_CK(cudaFuncSetAttribute(k_ls_fim_coop<kFimSmall, kFimSweeps>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       static_cast<int>(Fim<kFimSmall, kFimSweeps>::kSmem)));
+        INCRMT_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fim, kFimThreads, fsm));
         coop_blocks_fim = sms * (nb > 0 ? 1 : 0);
         INCRMT_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_ls_extrap_coop, kExtrapThreads, 0));
         coop_blocks_ext = sms * (nb > 0 ? 1 : 0);
@@ -659,17 +670,25 @@ int Sim::build_bands() {
     k_ls_mark_interface<<<gg, kB2, 0, stream>>>(lg, d_lso, wl);
     k_ls_dilate<true><<<gg, kB2, 0, stream>>>(lg, d_lso, wl, R);
     k_ls_dilate<false><<<gg, kB2, 0, stream>>>(lg, d_lso, wl, R);
-    k_ls_collect_candidates<<<gg, kB2, 0, stream>>>(lg, d_lso, wl, d_list, d_list_k, d_flags + 7, list_cap,
-                                                    d_flags + 10);
+    const dim3 gs(cdiv(32 * gg.x, kFimSmall), cdiv(8 * gg.y, kFimSmall), gg.z);
+    const bool small = static_cast<long>(gs.x) * gs.y * gs.z <= coop_blocks_fim;
+    if (small)
+        k_ls_collect_tiles<kFimSmall><<<gs, 256, 0, stream>>>(lg, d_lso, wl, d_list, d_list_k, d_flags + 7, list_cap,
+                                                              d_flags + 10);
+    else
+        k_ls_collect_tiles<kFimLarge><<<dim3(cdiv(32 * gg.x, kFimLarge), cdiv(8 * gg.y, kFimLarge), gg.z), 256, 0, stream>>>(
+            lg, d_lso, wl, d_list, d_list_k, d_flags + 7, list_cap, d_flags + 10);
     k_ls_fim_init<<<gg, kB2, 0, stream>>>(lg, d_lso, wl);
     launches += 8;
     INCRMT_CKL("level-set scan/newton/candidates");
     int maxs = kLsMaxSweeps, cap = list_cap;
     const int *countp = d_flags + 7;
     const LsObj *ob = d_lso;
-    void *args[] = {&lg, &ob, &d_list, &d_list_k, &countp, &cap, &d_flags, &maxs};
-    INCRMT_CK(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(k_ls_fim_coop), dim3(coop_blocks_fim), dim3(kFimThreads),
-                                          args, 0, stream));
+    void *args[] = {&lg, &ob, &wl, &d_list, &d_list_k, &countp, &cap, &d_flags, &maxs};
+    INCRMT_CK(cudaLaunchCooperativeKernel(small ? reinterpret_cast<void *>(k_ls_fim_coop<kFimSmall, kFimSweeps>)
+                                                : reinterpret_cast<void *>(k_ls_fim_coop<kFimLarge, kFimSweeps>),
+                                          dim3(coop_blocks_fim), dim3(kFimThreads), args,
+                                          small ? Fim<kFimSmall, kFimSweeps>::kSmem : Fim<kFimLarge, kFimSweeps>::kSmem, stream));
     launches++;
     INCRMT_CK(cudaMemcpyAsync(h_lsbox, d_lsbox, sizeof(int) * 4 * no, cudaMemcpyDeviceToHost, stream));
     int r = fetch_flags();
@@ -679,7 +698,8 @@ int Sim::build_bands() {
     ls_sweeps += h_flags[3];
     if (h_flags[12]) ls_monotone++;
     if (!h_flags[4]) { set_error("level-set march did not settle in %d sweeps", h_flags[3]); return INCRMT_ERR_NOCONV; }
-    k_ls_finish<<<gg, kB2, 0, stream>>>(lg, d_lso, wl);
+    const bool in_b = cdiv(h_flags[3], kFimSweeps) & 1;
+    k_ls_finish<<<gg, kB2, 0, stream>>>(lg, d_lso, wl, in_b);
     k_ls_trial<<<gg, kB2, 0, stream>>>(lg, d_lso, wl);
     k_ls_store_status<<<gg, kB2, 0, stream>>>(lg, d_lso, wl);
     launches += 3;
