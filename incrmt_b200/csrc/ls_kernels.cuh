@@ -659,9 +659,13 @@ __device__ __forceinline__ bool ls_candidate(const LsObj &o, int ij) {
     return (st == 0 || st == 7) && o.ia[ij];
 }
 
+/** Whether a status is that of a band point outside the solid. */
+__device__ __forceinline__ bool ls_outside(int st) { return st == 4 || st == 5; }
+
 /** Lists the tiles (TILE x TILE points of an object's window) that hold
- * candidates as (x | y << 16, object), one block of 256 threads per tile. */
-template <int TILE>
+ * candidates (OUTSIDE: points of the band outside the solid) as
+ * (x | y << 16, object), one block of 256 threads per tile. */
+template <int TILE, bool OUTSIDE>
 __global__ void k_ls_collect_tiles(LsGrid g, const LsObj *ob, const LsWin *win, int *list, int *list_k, int *count, int cap,
                                    int *overflow) {
     const LsWin w = win[blockIdx.z];
@@ -669,7 +673,8 @@ __global__ void k_ls_collect_tiles(LsGrid g, const LsObj *ob, const LsWin *win, 
     bool any = false;
     for (int t = threadIdx.x; t < TILE * TILE; t += blockDim.x) {
         const int i = w.x0 + blockIdx.x * TILE + t % TILE, j = w.y0 + blockIdx.y * TILE + t / TILE;
-        if (i < xe && j < ye && ls_candidate(ob[blockIdx.z], j * g.P + i)) any = true;
+        if (i < xe && j < ye && (OUTSIDE ? ls_outside(ob[blockIdx.z].s[j * g.P + i]) : ls_candidate(ob[blockIdx.z], j * g.P + i)))
+            any = true;
     }
     if (__syncthreads_or(any) && threadIdx.x == 0)
         ls_list_push(list, list_k, count, cap, overflow, blockIdx.x | blockIdx.y << 16, blockIdx.z);
@@ -862,8 +867,179 @@ __global__ void __launch_bounds__(kFimThreads, 1) k_ls_fim_coop(LsGrid g, const 
     }
 }
 
-/** All sweeps of the extrapolation wavefront in one cooperative launch (same
- * scheme as k_ls_fim_coop); flags[5] is raised for a singular fit. */
+/** The extrapolation's staging, as Fim: the fit reaches three points. */
+template <int TILE, int SWEEPS>
+struct Ext {
+    static constexpr int kHalo = 3 * SWEEPS, kReg = TILE + 2 * kHalo, kPoints = kReg * kReg, kRound = (kPoints + 31) & ~31;
+    // listed points: those a sweep may evaluate (three from the region's edge)
+    static constexpr int kList = (kReg - 6) * (kReg - 6);
+    static constexpr size_t kSmem = kPoints * 5 * sizeof(double) + kList * (3 * sizeof(double) + sizeof(short));
+};
+
+/** All sweeps of the extrapolation wavefront in one cooperative launch, staged
+ * like the march (k_ls_fim_coop): the fit's moments depend on the level set
+ * alone and are formed by the first sweep of a batch; the others only sum the
+ * values of the 7 x 7 window. A point whose window of radius 3 gives a singular
+ * fit raises flags[11]: the caller starts over with k_ls_extrap_coop, which
+ * widens the window. The first batch reads the reference map itself.
+ * flags[0..2], [3] and [4] as in k_ls_fim_coop.
+ *
+ * Bound by the window sums of the busiest SM. Measured (B200, us per call, one
+ * sweep per barrier over global memory -> here): rotor 128^2 266 -> 108, 1024^2
+ * 288 -> 107; 32 bodies 1024 x 2048 377 -> 271; flag 2048^2 469 -> 211. */
+template <int TILE, int SWEEPS>
+__global__ void __launch_bounds__(kFimThreads, 1) k_ls_extrap_tiles(LsGrid g, const LsObj *ob, const LsWin *win, const int *list,
+                                                                    const int *list_k, const int *countp, int cap, int *flags,
+                                                                    int max_sweeps) {
+    namespace cg = cooperative_groups;
+    cg::grid_group grid = cg::this_grid();
+    using E = Ext<TILE, SWEEPS>;
+    constexpr int REG = E::kReg, RR = E::kPoints, NL = E::kList;
+    extern __shared__ __align__(16) double ext_smem[];
+    double *ph = ext_smem, *xa = ph + RR, *ya = xa + RR, *xb = ya + RR, *yb = xb + RR, *fit = yb + RR;
+    unsigned short *work = reinterpret_cast<unsigned short *>(fit + 3 * NL);
+    __shared__ int nwork;
+    const int tid = threadIdx.x, count = min(*countp, cap);
+    bool done = false;
+    int it0 = 0;
+    for (int batch = 0; it0 < max_sweeps; batch++, it0 += SWEEPS) {
+        if (blockIdx.x == 0 && tid == 0) flags[(batch + 1) % 3] = 0;
+        const bool odd = batch & 1;
+        for (int tile = blockIdx.x; tile < count; tile += gridDim.x) {
+            const LsObj &o = ob[list_k[tile]];
+            const LsWin w = win[list_k[tile]];
+            const double *gx = batch == 0 ? o.nX : (odd ? o.b : o.a), *gy = batch == 0 ? o.nY : (odd ? o.d : o.c);
+            const int x0 = w.x0 + (list[tile] & 0xffff) * TILE - E::kHalo;
+            const int y0 = w.y0 + (list[tile] >> 16) * TILE - E::kHalo;
+            const int xe = min(w.x1, g.mL), ye = min(w.y1, g.nL);
+            __syncthreads();  // the tile before is written out
+            if (tid == 0) nwork = 0;
+            __syncthreads();
+            for (int t = tid; t < E::kRound; t += kFimThreads) {
+                const int lx = t % REG, ly = t / REG, i = x0 + lx, j = y0 + ly;
+                // points outside the band never enter a fit
+                double p = kUnset, x = 0, y = 0;
+                bool out = false;
+                if (t < RR && i >= 0 && i < g.mL && j >= 0 && j < g.nL) {
+                    const int ij = j * g.P + i, st = o.s[ij];
+                    if (st >= 2 && st <= 5) {
+                        out = ls_outside(st);
+                        p = o.phi[ij];
+                        x = out ? gx[ij] : o.nX[ij];
+                        y = out ? gy[ij] : o.nY[ij];
+                    }
+                }
+                if (t < RR) {
+                    ph[t] = p;
+                    xa[t] = xb[t] = x;
+                    ya[t] = yb[t] = y;
+                }
+                // (outside the window the band has no points of this object)
+                fim_push(out && lx >= 3 && lx < REG - 3 && ly >= 3 && ly < REG - 3, t, work, &nwork);
+            }
+            __syncthreads();
+            const int nw = nwork;
+            int mask = 0;
+#pragma unroll 1
+            for (int k = 0; k < SWEEPS; k++) {
+                const int ring = 3 * (k + 1);
+                const double *cx = k & 1 ? xb : xa, *cy = k & 1 ? yb : ya;
+                double *tx = k & 1 ? xa : xb, *ty = k & 1 ? ya : yb;
+                bool ch = false;
+                for (int t = tid; t < nw; t += kFimThreads) {
+                    const int q = work[t], lx = q % REG, ly = q / REG;
+                    if (lx < ring || lx >= REG - ring || ly < ring || ly >= REG - ring) continue;
+                    const double pp = ph[q];
+                    double acc[6] = {0, 0, 0, 0, 0, 0}, al, be, ga;
+                    if (k == 0) {
+                        // with the fit's moments (the loop of ls_extrap_point,
+                        // so that every sum rounds as there)
+                        double sw = 0, sx = 0, sy = 0, sxx = 0, sxy = 0, syy = 0;
+#pragma unroll
+                        for (int dj = -3; dj <= 3; dj++)
+#pragma unroll
+                            for (int di = -3; di <= 3; di++) {
+                                const int e = q + dj * REG + di;
+                                const double p = ph[e];
+                                if (!(p < pp)) continue;
+                                const double ww = pp - p;
+                                sw += ww;
+                                sx += di * ww;
+                                sy += dj * ww;
+                                sxx += di * di * ww;
+                                sxy += di * dj * ww;
+                                syy += dj * dj * ww;
+                                const double vx = cx[e], vy = cy[e];
+                                acc[0] += ww * vx; acc[1] += ww * di * vx; acc[2] += ww * dj * vx;
+                                acc[3] += ww * vy; acc[4] += ww * di * vy; acc[5] += ww * dj * vy;
+                            }
+                        double det = sw * (sxy * sxy - sxx * syy) + sx * sx * syy - 2 * sx * sxy * sy + sy * sy * sxx;
+                        if (fabs(det) < 1e-10) flags[11] = 1;
+                        det = 1 / det;
+                        al = (sxy * sxy - sxx * syy) * det; be = (sx * syy - sxy * sy) * det; ga = (sxx * sy - sxy * sx) * det;
+                        fit[t] = al;
+                        fit[NL + t] = be;
+                        fit[2 * NL + t] = ga;
+                    } else {
+#pragma unroll 1
+                        for (int dj = -3; dj <= 3; dj++)
+#pragma unroll
+                            for (int di = -3; di <= 3; di++) {
+                                const int e = q + dj * REG + di;
+                                const double p = ph[e];
+                                if (!(p < pp)) continue;
+                                const double ww = pp - p, vx = cx[e], vy = cy[e];
+                                acc[0] += ww * vx; acc[1] += ww * di * vx; acc[2] += ww * dj * vx;
+                                acc[3] += ww * vy; acc[4] += ww * di * vy; acc[5] += ww * dj * vy;
+                            }
+                        al = fit[t]; be = fit[NL + t]; ga = fit[2 * NL + t];
+                    }
+                    const double ox = acc[0] * al + acc[1] * be + acc[2] * ga, oy = acc[3] * al + acc[4] * be + acc[5] * ga;
+                    if ((ox != cx[q] || oy != cy[q]) && lx >= E::kHalo && lx < E::kHalo + TILE && ly >= E::kHalo &&
+                        ly < E::kHalo + TILE)
+                        ch = true;
+                    tx[q] = ox;
+                    ty[q] = oy;
+                }
+                if (__syncthreads_or(ch)) mask |= 1 << k;
+            }
+            if (mask && tid == 0) atomicOr(&flags[batch % 3], mask);
+            double *ox = odd ? o.a : o.b, *oy = odd ? o.c : o.d;
+            for (int t = tid; t < nw; t += kFimThreads) {
+                const int q = work[t], lx = q % REG, ly = q / REG, i = x0 + lx, j = y0 + ly;
+                if (lx >= E::kHalo && lx < E::kHalo + TILE && ly >= E::kHalo && ly < E::kHalo + TILE && i < xe && j < ye) {
+                    ox[j * g.P + i] = SWEEPS & 1 ? xb[q] : xa[q];
+                    oy[j * g.P + i] = SWEEPS & 1 ? yb[q] : ya[q];
+                }
+            }
+        }
+        grid.sync();
+        if (*reinterpret_cast<volatile int *>(&flags[11])) break;
+        const int mask = *reinterpret_cast<volatile int *>(&flags[batch % 3]);
+        const int last = __ffs(~mask) - 1;  // the first sweep that changed nothing
+        if (last < SWEEPS && it0 + last < max_sweeps) {
+            it0 += last + 1;
+            done = true;
+            break;
+        }
+    }
+    if (blockIdx.x == 0 && tid == 0) { flags[3] = done ? it0 : max_sweeps; flags[4] = done ? 1 : 0; }
+}
+
+/** Stores the values of k_ls_extrap_tiles (in o.b, o.d if in_b) into nX, nY. */
+__global__ void k_ls_extrap_keep(LsGrid g, const LsObj *ob, const LsWin *win, bool in_b) {
+    int i, j;
+    if (!ls_point(g, win, i, j)) return;
+    const LsObj &o = ob[blockIdx.z];
+    const int ij = j * g.P + i;
+    if (!ls_outside(o.s[ij])) return;
+    o.nX[ij] = in_b ? o.b[ij] : o.a[ij];
+    o.nY[ij] = in_b ? o.d[ij] : o.c[ij];
+}
+
+/** All sweeps of the extrapolation wavefront over global memory in one
+ * cooperative launch, each followed by a grid barrier, for fits that need a
+ * window wider than radius 3; flags[5] is raised where it stays singular. */
 __global__ void __launch_bounds__(kExtrapThreads, 1) k_ls_extrap_coop(LsGrid g, const LsObj *ob, const int *list, const int *list_k,
                                  const int *countp, int cap, int *flags, int max_sweeps) {
     namespace cg = cooperative_groups;

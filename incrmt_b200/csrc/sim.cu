@@ -28,6 +28,7 @@ inline dim3 g2(int m, int n) { return dim3(cdiv(m, 32), cdiv(n, 8)); }
  * share. Measured (B200, us per call, 16 against 32 wide): rotor 128^2 108 /
  * 149, 1024^2 283 / 163; 32 bodies 1024 x 2048 594 / 395; flag 2048^2 379 / 316. */
 constexpr int kFimSweeps = 4, kFimSmall = 16, kFimLarge = 32;
+constexpr int kExtSweeps = 3;           // of the extrapolation (k_ls_extrap_tiles)
 constexpr int kLsMaxSweeps = 400;       // cap of the fixed-point sweeps of one march
 constexpr int kExtrapMaxSweeps = 1000;  // cap of the extrapolation wavefront sweeps
 constexpr int kLearnedStrikes = 8;      // rejected learned guesses in a row ...
@@ -314,6 +315,13 @@ int Sim::create(const incrmt_grid *gr, const incrmt_phys *ph) {
                                        static_cast<int>(Fim<kFimSmall, kFimSweeps>::kSmem)));
         INCRMT_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fim, kFimThreads, fsm));
         coop_blocks_fim = sms * (nb > 0 ? 1 : 0);
+        const auto ext = k_ls_extrap_tiles<kFimLarge, kExtSweeps>;
+        constexpr size_t esm = Ext<kFimLarge, kExtSweeps>::kSmem;
+        INCRMT_CK(cudaFuncSetAttribute(ext, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(esm)));
+        INCRMT_CK(cudaFuncSetAttribute(k_ls_extrap_tiles<kFimSmall, kExtSweeps>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       static_cast<int>(Ext<kFimSmall, kExtSweeps>::kSmem)));
+        INCRMT_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ext, kFimThreads, esm));
+        if (nb == 0) coop_blocks_fim = 0;
         INCRMT_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_ls_extrap_coop, kExtrapThreads, 0));
         coop_blocks_ext = sms * (nb > 0 ? 1 : 0);
         if (coop_blocks_fim == 0 || coop_blocks_ext == 0) {
@@ -673,10 +681,10 @@ int Sim::build_bands() {
     const dim3 gs(cdiv(32 * gg.x, kFimSmall), cdiv(8 * gg.y, kFimSmall), gg.z);
     const bool small = static_cast<long>(gs.x) * gs.y * gs.z <= coop_blocks_fim;
     if (small)
-        k_ls_collect_tiles<kFimSmall><<<gs, 256, 0, stream>>>(lg, d_lso, wl, d_list, d_list_k, d_flags + 7, list_cap,
+        k_ls_collect_tiles<kFimSmall, false><<<gs, 256, 0, stream>>>(lg, d_lso, wl, d_list, d_list_k, d_flags + 7, list_cap,
                                                               d_flags + 10);
     else
-        k_ls_collect_tiles<kFimLarge><<<dim3(cdiv(32 * gg.x, kFimLarge), cdiv(8 * gg.y, kFimLarge), gg.z), 256, 0, stream>>>(
+        k_ls_collect_tiles<kFimLarge, false><<<dim3(cdiv(32 * gg.x, kFimLarge), cdiv(8 * gg.y, kFimLarge), gg.z), 256, 0, stream>>>(
             lg, d_lso, wl, d_list, d_list_k, d_flags + 7, list_cap, d_flags + 10);
     k_ls_fim_init<<<gg, kB2, 0, stream>>>(lg, d_lso, wl);
     launches += 8;
@@ -721,31 +729,56 @@ int Sim::pin() {
 }
 
 /** levelset::extrapolate_fields for every object (traverse.hh:235-260),
- * the objects' wavefronts settling together in one cooperative launch. */
+ * the objects' wavefronts settling together in one cooperative launch: in
+ * staged tiles, or (a fit that needs a wider window) over global memory. */
 int Sim::extrapolate_all() {
     const int no = static_cast<int>(obj.size());
     if (no == 0) return INCRMT_OK;
-    INCRMT_CK(cudaMemsetAsync(d_flags, 0, sizeof(int) * 11, stream));
-    k_ls_collect_outside<<<wgrid(1), kB2, 0, stream>>>(lg, d_lso, win(1), d_list, d_list_k, d_flags + 7,
-                                                       list_cap, d_flags + 10);
-    k_ls_extrap_init<<<4 * kB200SMs, 256, 0, stream>>>(d_lso, d_list, d_list_k, d_flags + 7, list_cap);
-    launches += 2;
-    INCRMT_CKL("collect");
+    INCRMT_CK(cudaMemsetAsync(d_flags, 0, sizeof(int) * 12, stream));
+    const dim3 gg = wgrid(1);
+    const LsWin *wl = win(1);
     int maxs = kExtrapMaxSweeps, cap = list_cap;
     const int *countp = d_flags + 7;
     const LsObj *ob = d_lso;
-    void *args[] = {&lg, &ob, &d_list, &d_list_k, &countp, &cap, &d_flags, &maxs};
-    INCRMT_CK(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(k_ls_extrap_coop), dim3(coop_blocks_ext),
-                                          dim3(kExtrapThreads), args, 0, stream));
+    const dim3 gs(cdiv(32 * gg.x, kFimSmall), cdiv(8 * gg.y, kFimSmall), gg.z);
+    const bool small = static_cast<long>(gs.x) * gs.y * gs.z <= coop_blocks_fim;
+    if (small)
+        k_ls_collect_tiles<kFimSmall, true><<<gs, 256, 0, stream>>>(lg, d_lso, wl, d_list, d_list_k, d_flags + 7, list_cap,
+                                                                    d_flags + 10);
+    else
+        k_ls_collect_tiles<kFimLarge, true>
+            <<<dim3(cdiv(32 * gg.x, kFimLarge), cdiv(8 * gg.y, kFimLarge), gg.z), 256, 0, stream>>>(
+                lg, d_lso, wl, d_list, d_list_k, d_flags + 7, list_cap, d_flags + 10);
+    launches++;
+    INCRMT_CKL("collect");
+    void *targs[] = {&lg, &ob, &wl, &d_list, &d_list_k, &countp, &cap, &d_flags, &maxs};
+    INCRMT_CK(cudaLaunchCooperativeKernel(small ? reinterpret_cast<void *>(k_ls_extrap_tiles<kFimSmall, kExtSweeps>)
+                                                : reinterpret_cast<void *>(k_ls_extrap_tiles<kFimLarge, kExtSweeps>),
+                                          dim3(coop_blocks_fim), dim3(kFimThreads), targs,
+                                          small ? Ext<kFimSmall, kExtSweeps>::kSmem : Ext<kFimLarge, kExtSweeps>::kSmem, stream));
     launches++;
     int r = fetch_flags();
     if (r) return r;
+    const bool wide = h_flags[11] != 0;
+    if (wide) {
+        INCRMT_CK(cudaMemsetAsync(d_flags, 0, sizeof(int) * 12, stream));
+        k_ls_collect_outside<<<gg, kB2, 0, stream>>>(lg, d_lso, wl, d_list, d_list_k, d_flags + 7, list_cap, d_flags + 10);
+        k_ls_extrap_init<<<4 * kB200SMs, 256, 0, stream>>>(d_lso, d_list, d_list_k, d_flags + 7, list_cap);
+        launches += 2;
+        INCRMT_CKL("collect");
+        void *args[] = {&lg, &ob, &d_list, &d_list_k, &countp, &cap, &d_flags, &maxs};
+        INCRMT_CK(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(k_ls_extrap_coop), dim3(coop_blocks_ext),
+                                              dim3(kExtrapThreads), args, 0, stream));
+        launches++;
+        if ((r = fetch_flags())) return r;
+    }
     if (h_flags[5]) { set_error("singular extrapolation fit"); return h_flags[5]; }
     if (h_flags[10]) { set_error("extrapolation list overflow"); return INCRMT_ERR_BADARG; }
     ex_sweeps += h_flags[3];
     if (!h_flags[4]) { set_error("extrapolation did not settle in %d sweeps", h_flags[3]); return INCRMT_ERR_NOCONV; }
     // After the last sweep both buffers hold the same values.
-    k_ls_extrap_store<<<4 * kB200SMs, 256, 0, stream>>>(d_lso, d_list, d_list_k, d_flags + 7, list_cap);
+    if (wide) k_ls_extrap_store<<<4 * kB200SMs, 256, 0, stream>>>(d_lso, d_list, d_list_k, d_flags + 7, list_cap);
+    else k_ls_extrap_keep<<<gg, kB2, 0, stream>>>(lg, d_lso, wl, cdiv(h_flags[3], kExtSweeps) & 1);
     launches++;
     INCRMT_CKL("k_ls_extrap_store");
     return INCRMT_OK;
