@@ -203,7 +203,9 @@ __global__ void k_galerkin(Op op, int fm, int fn, int px, int py, bool kx, bool 
     for (int e = 0; e < 9; e++) st[e * N + colour_index(cm, cn, I, J)] = q[e];
 }
 
-/** k_galerkin for a 32 x 8 tile of coarse unknowns per 256-thread block,
+constexpr int kGalRows = 4;  // coarse rows of a tile
+
+/** k_galerkin for a 32 x kGalRows tile of coarse unknowns per block,
  * with every input staged in shared memory first: the nine stencil entries
  * of the fine points of the tile's supports (coef9; the fine region
  * 2X0-1 .. 2(X0+31)+1 in a coarsened direction, X0 .. X0+31 otherwise) and
@@ -211,16 +213,22 @@ __global__ void k_galerkin(Op op, int fm, int fn, int px, int py, bool kx, bool 
  * stencil neighbours), zero outside a non-periodic grid. The sums then run
  * exactly as in k_galerkin, in the same order: the same values, without
  * each thread re-reading some four hundred entries from global memory.
- * Dynamic shared memory: galerkin_tile_smem(kx, ky) bytes. */
+ * Dynamic shared memory: galerkin_tile_smem(kx, ky) bytes.
+ *
+ * Bound by the sums' shared-memory reads and FP64 latency. Four rows leave room
+ * for three blocks per SM, and the sums have no branches: a point's zero
+ * weights are known from its parities. Measured (B200, us; 8 rows, tests of
+ * every weight -> here): MAC 4096^2 1782 -> 848 (8 rows 1163, 2 rows 1044), the
+ * 2048^2 flag's Galerkin levels 42.1 -> 18.7, FEM 1024^2 152 -> 57. */
 template <class Op, bool KX, bool KY>
-__global__ void __launch_bounds__(256) k_galerkin_tile(Op op, int fm, int fn, int px, int py, int cm, int cn,
+__global__ void __launch_bounds__(32 * kGalRows) k_galerkin_tile(Op op, int fm, int fn, int px, int py, int cm, int cn,
                                                        double *st, const double *P) {
     // The coarsening flags are template parameters: with them every loop
     // below has fixed bounds and every offset of a support point or stencil
     // neighbour relative to the coarse point is a constant, so the nine sums
     // stay in registers (indexed at run time they would live in local memory).
     extern __shared__ __align__(16) double gal_smem[];
-    constexpr int CTW = 32, CTH = 8;
+    constexpr int CTW = 32, CTH = kGalRows;
     constexpr bool kx = KX, ky = KY;
     const int X0 = blockIdx.x * CTW, Y0 = blockIdx.y * CTH;
     const int SX0 = kx ? 2 * X0 - 1 : X0, SY0 = ky ? 2 * Y0 - 1 : Y0;
@@ -250,9 +258,9 @@ __global__ void __launch_bounds__(256) k_galerkin_tile(Op op, int fm, int fn, in
         const int xu = SX0 + t % SW, yu = SY0 + t / SW;
         bool ok = xu <= sxmax && yu <= symax;
         const int i = wrap_idx(xu, fm, px, ok), j = wrap_idx(yu, fn, py, ok);
-        if (!ok) continue;  // outside the grid (weight zero) or no support of the tile: never read
-        double a[9];
-        op.coef9(i, j, a);
+        // outside the grid (weight zero) or no support of the tile: zero
+        double a[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+        if (ok) op.coef9(i, j, a);
 #pragma unroll
         for (int k = 0; k < 9; k++) As[k * SA + t] = a[k];
     }
@@ -262,34 +270,37 @@ __global__ void __launch_bounds__(256) k_galerkin_tile(Op op, int fm, int fn, in
     double q[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     // Support points fi = 2I-1+u (u = 0..2) in a coarsened direction, fi = I
     // otherwise; visited in the order of k_galerkin (rows, then columns).
-    // Relative to I: base_of(fi) - I = floor((u-1)/2) there, 0 otherwise.
-    const int x0 = kx ? 2 * I - 1 : I, y0 = ky ? 2 * J - 1 : J;
+    // Which of a point's weights can differ from zero is known from its
+    // parities (a point on a coarse point has the single weight 1), so the sums
+    // run without a branch; a weight or entry that is zero all the same adds
+    // zero.
+    const double *ac = As + (kx ? 2 : 1) * (threadIdx.x & 31) + SW * (ky ? 2 : 1) * (threadIdx.x >> 5);
+    const double *pc = Ps + 4 * (1 + (kx ? 2 : 1) * (threadIdx.x & 31) + NW * (1 + (ky ? 2 : 1) * (threadIdx.x >> 5)));
 #pragma unroll
     for (int v = 0; v <= (ky ? 2 : 0); v++)
 #pragma unroll
         for (int u = 0; u <= (kx ? 2 : 0); u++) {
-            const int fi = x0 + u, fj = y0 + v;
-            // pweight(fi, fj, I, J) from the staged weights
-            const int qx = kx ? -((u - 1) >> 1) : 0, qy = ky ? -((v - 1) >> 1) : 0;
-            if (qx < 0 || qx > 1 || qy < 0 || qy > 1) continue;
-            const double w = Ps[4 * ((fi - NX0) + NW * (fj - NY0)) + qx + 2 * qy];
-            if (w == 0) continue;
-            const int ls = (fi - SX0) + SW * (fj - SY0);
+            // this support point's weight for the coarse point
+            const int qx = kx && u == 0, qy = ky && v == 0;
+            const bool on_x = !kx || u == 1, on_y = !ky || v == 1;  // on the coarse point's column / row
+            const double w = on_x && on_y ? 1.0 : pc[4 * (u + NW * v) + qx + 2 * qy];
 #pragma unroll
             for (int dj = -1; dj <= 1; dj++)
 #pragma unroll
                 for (int di = -1; di <= 1; di++) {
-                    const double av = As[(3 * (dj + 1) + di + 1) * SA + ls];
-                    if (av == 0) continue;
-                    const double *g = Ps + 4 * ((fi + di - NX0) + NW * (fj + dj - NY0));
+                    if (Op::kFivePoint && di != 0 && dj != 0) continue;
+                    const double wa = __dmul_rn(w, ac[(3 * (dj + 1) + di + 1) * SA + u + SW * v]);
+                    const double *g = pc + 4 * (u + di + NW * (v + dj));
                     const int ox = kx ? ((u - 1 + di) >> 1) : di, oy = ky ? ((v - 1 + dj) >> 1) : dj;
+                    const bool gx = kx && ((u - 1 + di) & 1), gy = ky && ((v - 1 + dj) & 1);  // between coarse columns / rows
 #pragma unroll
                     for (int r = 0; r < 4; r++) {
                         const int kx_ = ox + (r & 1), ky_ = oy + (r >> 1);
+                        if (((r & 1) && !gx) || ((r >> 1) && !gy)) continue;
                         if (kx_ < -1 || kx_ > 1 || ky_ < -1 || ky_ > 1) continue;
-                        if (g[r] == 0) continue;
                         double &qe = q[3 * (ky_ + 1) + kx_ + 1];
-                        qe = add_prod(qe, __dmul_rn(w, av), g[r]);
+                        // (outside a non-periodic grid the staged weight is 0)
+                        qe = add_prod(qe, wa, g[r]);
                     }
                 }
         }
@@ -313,7 +324,7 @@ cudaError_t set_galerkin_attr(int bytes) {
 
 /** Shared memory of k_galerkin_tile for the coarsening flags. */
 inline size_t galerkin_tile_smem(bool kx, bool ky) {
-    const int SW = kx ? 65 : 32, SH = ky ? 17 : 8;
+    const int SW = kx ? 65 : 32, SH = ky ? 2 * kGalRows + 1 : kGalRows;
     return sizeof(double) * (9 * SW * SH + 4 * (SW + 2) * (SH + 2));
 }
 
@@ -1276,18 +1287,18 @@ int Multigrid::set_unit_density() {
 int Multigrid::galerkin_all() {
     for (size_t l = 1; l < lev.size(); l++) {
         MgLevel &F = lev[l - 1], &C = lev[l];
-        const dim3 gf = grid2(F.m, F.n), gc = grid2(C.m, C.n), gt(cdiv(C.m, 32), cdiv(C.n, 8));
+        const dim3 gf = grid2(F.m, F.n), gc = grid2(C.m, C.n), gt(cdiv(C.m, 32), cdiv(C.n, kGalRows));
         const size_t gsm = galerkin_tile_smem(F.kx, F.ky);
         auto build = [&](auto op) {
             for (int pass = 0; pass < 2; pass++)
                 k_build_p<<<gf, kBlk2, 0, stream>>>(op, F.m, F.n, px, py, F.kx, F.ky, C.m, C.n, F.P, pass);
             using OpT = decltype(op);
             if (tiles && F.kx && F.ky)
-                k_galerkin_tile<OpT, true, true><<<gt, 256, gsm, stream>>>(op, F.m, F.n, px, py, C.m, C.n, C.st, F.P);
+                k_galerkin_tile<OpT, true, true><<<gt, 32 * kGalRows, gsm, stream>>>(op, F.m, F.n, px, py, C.m, C.n, C.st, F.P);
             else if (tiles && F.kx)
-                k_galerkin_tile<OpT, true, false><<<gt, 256, gsm, stream>>>(op, F.m, F.n, px, py, C.m, C.n, C.st, F.P);
+                k_galerkin_tile<OpT, true, false><<<gt, 32 * kGalRows, gsm, stream>>>(op, F.m, F.n, px, py, C.m, C.n, C.st, F.P);
             else if (tiles)
-                k_galerkin_tile<OpT, false, true><<<gt, 256, gsm, stream>>>(op, F.m, F.n, px, py, C.m, C.n, C.st, F.P);
+                k_galerkin_tile<OpT, false, true><<<gt, 32 * kGalRows, gsm, stream>>>(op, F.m, F.n, px, py, C.m, C.n, C.st, F.P);
             else
                 k_galerkin<<<gc, kBlk2, 0, stream>>>(op, F.m, F.n, px, py, F.kx, F.ky, C.m, C.n, C.st, F.P);
         };
