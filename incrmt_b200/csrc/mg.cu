@@ -41,19 +41,6 @@ __host__ __device__ __forceinline__ int half_floor(int a) { return a >= 0 ? a / 
  * when the direction is coarsened, else i. */
 __host__ __device__ __forceinline__ int base_of(int i, bool k) { return k ? half_floor(i) : i; }
 
-/** Coarse index of corner q (0 or 1) above base B along a direction of
- * coarse size mc, or -1 outside a non-periodic grid (and for q=1 when the
- * direction is not coarsened). */
-__host__ __device__ __forceinline__ int corner_of(int B, int q, int mc, int p, bool k) {
-    if (!k && q) return -1;
-    int c = B + q;
-    if (c < 0 || c >= mc) {
-        if (!p) return -1;
-        c = (c % mc + mc) % mc;
-    }
-    return c;
-}
-
 /** Prolongation weight of fine point (fi,fj) (unwrapped indices) for coarse
  * point (I,J): entry qx+2qy of the point's four stored weights, with (qx,qy)
  * the coarse point's offset from the point's base; 0 when it is not one of
@@ -68,6 +55,15 @@ __device__ __forceinline__ double pweight(const W *P, int fm, int fn, int px, in
     if (!ok) return 0;
     return static_cast<double>(P[4 * (static_cast<long>(i) + static_cast<long>(fm) * j) + qx + 2 * qy]);
 }
+
+}  // namespace
+}  // namespace incrmt
+
+#include "mg_transfer.cuh"
+
+namespace incrmt {
+
+namespace {
 
 inline bool can_coarsen(int m, int p) { return p ? (m % 2 == 0 && m / 2 >= 4) : m >= 5; }
 
@@ -103,65 +99,6 @@ __global__ void k_fem_coef(const double *rho, int ml, int mf, int nf, double *c,
     cf[j * mf + i] = static_cast<float>(v);
 }
 
-
-/** Operator-dependent prolongation of a level (black-box multigrid:
- * Dendy, J. Comput. Phys. 48 (1982) 366-386): four weights per fine point,
- * P[4f+qx+2qy] for the coarse point at offset (qx,qy) from the point's base
- * (base_of). A point on a coarse point takes it with weight 1; a point
- * between two coarse points along x takes L/(-C) and R/(-C), L, C, R its
- * stencil summed over the columns left of, through and right of it (the
- * operator collapsed along y), and along y likewise with the rows; a point
- * between four coarse points takes -(its stencil entries times its eight
- * neighbours' weights)/(its diagonal), so pass 1 runs after pass 0 has set
- * the others. Constant coefficients give the bilinear 1, 1/2, 1/4; across a
- * density jump the weights follow the flux; at the zero-pressure edge of the
- * MAC system the last point's weight drops to about 1/3. Weights stay in
- * double precision so that constants map onto constants exactly and the
- * coarse operators of a pure-Neumann problem keep their null space. */
-template <class Op>
-__global__ void k_build_p(Op op, int fm, int fn, int px, int py, bool kx, bool ky, int cm, int cn, double *P,
-                          int pass) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= fm || j >= fn) return;
-    const bool xo = kx && (i & 1), yo = ky && (j & 1);
-    if ((pass == 1) != (xo && yo)) return;
-    double a[9];
-    op.coef9(i, j, a);
-    double *q = P + 4 * (static_cast<long>(i) + static_cast<long>(fm) * j);
-    double w[4] = {0, 0, 0, 0};
-    const int bx = base_of(i, kx), by = base_of(j, ky);
-    const bool v1 = corner_of(bx, 1, cm, px, kx) >= 0, v2 = corner_of(by, 1, cn, py, ky) >= 0;
-    if (!xo && !yo) {
-        w[0] = 1;
-    } else if (xo && !yo) {
-        const double L = a[0] + a[3] + a[6], C = a[1] + a[4] + a[7], R = a[2] + a[5] + a[8];
-        w[0] = L / (-C);
-        if (v1) w[1] = R / (-C);
-    } else if (!xo && yo) {
-        const double D = a[0] + a[1] + a[2], M = a[3] + a[4] + a[5], U = a[6] + a[7] + a[8];
-        w[0] = D / (-M);
-        if (v2) w[2] = U / (-M);
-    } else {
-        double acc[4] = {0, 0, 0, 0};
-        for (int dj = -1; dj <= 1; dj++)
-            for (int di = -1; di <= 1; di++) {
-                const double av = a[3 * (dj + 1) + di + 1];
-                if ((di == 0 && dj == 0) || av == 0) continue;
-                bool ok = true;
-                const int gi = wrap_idx(i + di, fm, px, ok), gj = wrap_idx(j + dj, fn, py, ok);
-                if (!ok) continue;
-                const double *g = P + 4 * (static_cast<long>(gi) + static_cast<long>(fm) * gj);
-                const int ox = base_of(i + di, kx) - bx, oy = base_of(j + dj, ky) - by;
-                for (int r = 0; r < 4; r++) {
-                    const int cx = ox + (r & 1), cy = oy + (r >> 1);
-                    if (g[r] != 0 && cx <= 1 && cy <= 1) acc[cx + 2 * cy] = add_prod(acc[cx + 2 * cy], av, g[r]);
-                }
-            }
-        for (int r = 0; r < 4; r++)
-            if (((r & 1) == 0 || v1) && ((r >> 1) == 0 || v2)) w[r] = -acc[r] / a[4];
-    }
-    q[0] = w[0]; q[1] = w[1]; q[2] = w[2]; q[3] = w[3];
-}
 
 /** Galerkin coarse stencil A_c = P^T A P, one thread per coarse unknown
  * (I,J): over the fine points f of its support (the 3 x 3 fine points about
@@ -517,88 +454,6 @@ __global__ void k_restrict(Op op, const T *z, const T *b, int fm, int fn, int px
         }
     bc[I + cm * J] = t;
     zc[I + cm * J] = 0;
-}
-
-/** k_restrict for a 32 x 8 tile of coarse unknowns per 256-thread block,
- * each fine residual computed once: the block first evaluates b - A z at
- * every fine unknown of its coarse points' supports (the fine region
- * 2X0-1 .. 2(X0+31)+1 in a coarsened direction, X0 .. X0+31 otherwise) into
- * shared memory, then every coarse point sums its support's residuals with
- * the weights and in the order of k_restrict: the same values. */
-template <class Op, class T, bool KX, bool KY>
-__global__ void __launch_bounds__(256) k_restrict_tile(Op op, const T *z, const T *b, int fm, int fn, int px, int py,
-                                                       int cm, int cn, T *bc, T *zc, const double *P) {
-    // The coarsening flags are template parameters, so the region's width
-    // (the divisor of the staging loop's index) is a constant.
-    constexpr bool kx = KX, ky = KY;
-    constexpr int CTW = 32, CTH = 8, RW = 2 * CTW + 1, RH = 2 * CTH + 1;
-    __shared__ T rs[RW * RH];
-    __shared__ double ps[4 * RW * RH];  // the region's prolongation weights (zero outside the grid)
-    const int X0 = blockIdx.x * CTW, Y0 = blockIdx.y * CTH;
-    const int FX0 = kx ? 2 * X0 - 1 : X0, FY0 = ky ? 2 * Y0 - 1 : Y0;
-    constexpr int FW = kx ? RW : CTW, FH = ky ? RH : CTH;
-    // Only fine unknowns in the support of a coarse point I < cm, J < cn are
-    // needed (and beyond them a periodic index could wrap past the grid).
-    const int fxmax = kx ? 2 * cm - 1 : cm - 1, fymax = ky ? 2 * cn - 1 : cn - 1;
-    for (int t = threadIdx.x; t < FW * FH; t += blockDim.x) {
-        const int fxu = FX0 + t % FW, fyu = FY0 + t / FW;
-        bool ok = fxu <= fxmax && fyu <= fymax;
-        const int fx = wrap_idx(fxu, fm, px, ok), fy = wrap_idx(fyu, fn, py, ok);
-        T r = 0;
-        double w0 = 0, w1 = 0, w2 = 0, w3 = 0;
-        if (ok) {
-            const int f = fx + fm * fy;
-            r = residual_at(op, fx, fy, z, b[f]);
-            // four weights per fine point: 32-byte aligned, two 16-byte loads
-            const double2 *q = reinterpret_cast<const double2 *>(P + 4 * static_cast<long>(f));
-            const double2 q01 = q[0], q23 = q[1];
-            w0 = q01.x; w1 = q01.y; w2 = q23.x; w3 = q23.y;
-        }
-        rs[t] = r;
-        ps[4 * t] = w0; ps[4 * t + 1] = w1; ps[4 * t + 2] = w2; ps[4 * t + 3] = w3;
-    }
-    __syncthreads();
-    const int I = X0 + (threadIdx.x & 31), J = Y0 + (threadIdx.x >> 5);
-    if (I >= cm || J >= cn) return;
-    // The support in k_restrict's order, each fine point read from its
-    // (unwrapped) position in the staged region.
-    const int x0 = kx ? 2 * I - 1 : I, x1 = kx ? 2 * I + 1 : I, y0 = ky ? 2 * J - 1 : J, y1 = ky ? 2 * J + 1 : J;
-    T t = 0;
-    for (int fj = y0; fj <= y1; fj++)
-        for (int fi = x0; fi <= x1; fi++) {
-            // pweight(fi, fj, I, J) from the staged weights
-            const int qx = I - base_of(fi, kx), qy = J - base_of(fj, ky);
-            if (qx < 0 || qx > 1 || qy < 0 || qy > 1) continue;
-            const int lt = (fi - FX0) + FW * (fj - FY0);
-            const T w = static_cast<T>(ps[4 * lt + qx + 2 * qy]);
-            if (w == 0) continue;
-            t = add_prod(t, w, rs[lt]);
-        }
-    bc[I + cm * J] = t;
-    zc[I + cm * J] = 0;
-}
-
-/** Fine correction z_f += P z_c, from the point's four stored weights. */
-template <class T>
-__global__ void k_prolong(T *zf, int fm, int fn, int px, int py, bool kx, bool ky,
-                          const T *zc, int cm, int cn, const double *P) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= fm || j >= fn) return;
-    const long f = i + static_cast<long>(fm) * j;
-    const double2 *q2 = reinterpret_cast<const double2 *>(P + 4 * f);  // 32-byte aligned
-    const double2 q01 = q2[0], q23 = q2[1];
-    const double q[4] = {q01.x, q01.y, q23.x, q23.y};
-    const int bx = base_of(i, kx), by = base_of(j, ky);
-    T t = 0;
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-        const double w = q[r];
-        if (w == 0) continue;
-        const int I = corner_of(bx, r & 1, cm, px, kx), J = corner_of(by, r >> 1, cn, py, ky);
-        if (I < 0 || J < 0) continue;  // k_build_p leaves such corners at 0
-        t = add_prod(t, static_cast<T>(w), zc[I + cm * J]);
-    }
-    zf[f] += t;
 }
 
 /** Coarsest-level solve: `sweeps` four-colour Gauss-Seidel sweeps by one
@@ -1026,23 +881,31 @@ int smooth(Op op, T *z, T *zalt, const T *b, int m, int n, int sweeps, cudaStrea
     return INCRMT_OK;
 }
 
-/** Coarse right-hand side and cleared coarse iterate: the tiled restriction,
- * or k_restrict when tiles are off (the identity check of
+/** Coarse right-hand side and cleared coarse iterate: the restriction by
+ * cells, or k_restrict when tiles are off (the identity check of
  * incrmt_mg_set_tiles covers both). */
 template <class Op, class T>
-void restrict_launch(bool tiles, Op op, cudaStream_t s, const T *z, const T *b, int fm, int fn, int px, int py,
-                     bool kx, bool ky, int cm, int cn, T *bc, T *zc, const double *we) {
+void restrict_launch(bool tiles, Op op, cudaStream_t s, const T *z, const T *b, int px, int py, const MgLevel &L,
+                     const MgLevel &C, T *bc, T *zc, const T *Q) {
+    const int fm = L.m, fn = L.n, cm = C.m, cn = C.n;
     if (!tiles) {
-        k_restrict<<<grid2(cm, cn), kBlk2, 0, s>>>(op, z, b, fm, fn, px, py, kx, ky, cm, cn, bc, zc, we);
+        k_restrict<<<grid2(cm, cn), kBlk2, 0, s>>>(op, z, b, fm, fn, px, py, L.kx, L.ky, cm, cn, bc, zc, L.P);
         return;
     }
-    const dim3 g(cdiv(cm, 32), cdiv(cn, 8));
-    if (kx && ky)
-        k_restrict_tile<Op, T, true, true><<<g, 256, 0, s>>>(op, z, b, fm, fn, px, py, cm, cn, bc, zc, we);
-    else if (kx)
-        k_restrict_tile<Op, T, true, false><<<g, 256, 0, s>>>(op, z, b, fm, fn, px, py, cm, cn, bc, zc, we);
-    else
-        k_restrict_tile<Op, T, false, true><<<g, 256, 0, s>>>(op, z, b, fm, fn, px, py, cm, cn, bc, zc, we);
+    const dim3 g(cdiv(cm, L.kx ? kRX - 1 : kRX), cdiv(cn, L.ky ? kRY - 1 : kRY)), t(kRX, kRY);
+    if (L.kx && L.ky) k_restrict_cells<Op, T, true, true><<<g, t, 0, s>>>(op, z, b, fm, fn, px, py, cm, cn, bc, zc, Q);
+    else if (L.kx) k_restrict_cells<Op, T, true, false><<<g, t, 0, s>>>(op, z, b, fm, fn, px, py, cm, cn, bc, zc, Q);
+    else k_restrict_cells<Op, T, false, true><<<g, t, 0, s>>>(op, z, b, fm, fn, px, py, cm, cn, bc, zc, Q);
+}
+
+/** z += P z_c. */
+template <class T>
+void prolong_launch(cudaStream_t s, T *z, int px, int py, const MgLevel &L, const MgLevel &C, const T *zc, const T *Q) {
+    const dim3 g = grid2(cells_of(L.m, L.kx), cells_of(L.n, L.ky));
+    const bool vec = L.m % 2 == 0 && reinterpret_cast<uintptr_t>(z) % (2 * sizeof(T)) == 0;
+    if (L.kx && L.ky) k_prolong_cells<T, true, true><<<g, kBlk2, 0, s>>>(z, L.m, L.n, px, py, zc, C.m, C.n, Q, vec);
+    else if (L.kx) k_prolong_cells<T, true, false><<<g, kBlk2, 0, s>>>(z, L.m, L.n, px, py, zc, C.m, C.n, Q, vec);
+    else k_prolong_cells<T, false, true><<<g, kBlk2, 0, s>>>(z, L.m, L.n, px, py, zc, C.m, C.n, Q, vec);
 }
 
 }  // namespace
@@ -1150,6 +1013,8 @@ int Multigrid::build_hierarchy() {
     for (size_t l = 0; l + 1 < lev.size(); l++) {
         INCRMT_CK(cudaMalloc(&lev[l].P, sizeof(double) * 4 * lev[l].N));
         INCRMT_CK(cudaMemsetAsync(lev[l].P, 0, sizeof(double) * 4 * lev[l].N, stream));
+        INCRMT_CK(cudaMalloc(&lev[l].Q, (sizeof(double) + sizeof(float)) * lev[l].planes()));
+        lev[l].Qf = reinterpret_cast<float *>(lev[l].Q + lev[l].planes());
     }
     if (lev.size() > 1 && lev.back().N <= kDirectMax) {
         const long N = lev.back().N;
@@ -1180,7 +1045,7 @@ int Multigrid::build_hierarchy() {
 void Multigrid::destroy() {
     for (auto &L : lev) {
         cudaFree(L.z); cudaFree(L.b); cudaFree(L.st); cudaFree(L.zf); cudaFree(L.bf); cudaFree(L.stf);
-        cudaFree(L.z2); cudaFree(L.zf2); cudaFree(L.P);
+        cudaFree(L.z2); cudaFree(L.zf2); cudaFree(L.P); cudaFree(L.Q);
     }
     lev.clear();
     cudaFree(ex); cudaFree(ey); cudaFree(exf); cudaFree(eyf); cudaFree(c); cudaFree(cf);
@@ -1287,12 +1152,16 @@ int Multigrid::set_unit_density() {
 int Multigrid::galerkin_all() {
     for (size_t l = 1; l < lev.size(); l++) {
         MgLevel &F = lev[l - 1], &C = lev[l];
-        const dim3 gf = grid2(F.m, F.n), gc = grid2(C.m, C.n), gt(cdiv(C.m, 32), cdiv(C.n, kGalRows));
+        const dim3 gc = grid2(C.m, C.n), gt(cdiv(C.m, 32), cdiv(C.n, kGalRows));
         const size_t gsm = galerkin_tile_smem(F.kx, F.ky);
         auto build = [&](auto op) {
-            for (int pass = 0; pass < 2; pass++)
-                k_build_p<<<gf, kBlk2, 0, stream>>>(op, F.m, F.n, px, py, F.kx, F.ky, C.m, C.n, F.P, pass);
             using OpT = decltype(op);
+            const int cx = cells_of(F.m, F.kx), cy = cells_of(F.n, F.ky);
+            const bool both = F.kx && F.ky;
+            const dim3 gb(cdiv(cx, both ? kPX - 1 : kPX), cdiv(cy, both ? kPY - 1 : kPY)), tb(kPX, kPY);
+            if (both) k_build_p<OpT, true, true><<<gb, tb, 0, stream>>>(op, F.m, F.n, px, py, C.m, C.n, F.P, F.Q);
+            else if (F.kx) k_build_p<OpT, true, false><<<gb, tb, 0, stream>>>(op, F.m, F.n, px, py, C.m, C.n, F.P, F.Q);
+            else k_build_p<OpT, false, true><<<gb, tb, 0, stream>>>(op, F.m, F.n, px, py, C.m, C.n, F.P, F.Q);
             if (tiles && F.kx && F.ky)
                 k_galerkin_tile<OpT, true, true><<<gt, 32 * kGalRows, gsm, stream>>>(op, F.m, F.n, px, py, C.m, C.n, C.st, F.P);
             else if (tiles && F.kx)
@@ -1310,7 +1179,7 @@ int Multigrid::galerkin_all() {
             GenOp<double> g; g.m = F.m; g.n = F.n; g.px = px; g.py = py; g.N = F.N; g.st = F.st;
             build(g);
         }
-        launches += 3;
+        launches += 2;
         INCRMT_CKL("galerkin");
     }
     f32_stale = true;
@@ -1360,6 +1229,11 @@ int Multigrid::cast_levels() {
         k_cast_stencil<<<cdiv(C.N, 256) < kRedBlocks ? cdiv(C.N, 256) : kRedBlocks, 256, 0, stream>>>(C.st, C.stf, C.N);
         launches++;
     }
+    for (size_t l = 0; l + 1 < lev.size(); l++) {
+        const long N = lev[l].planes();
+        k_cast_planes<<<cdiv(N, 256) < kRedBlocks ? cdiv(N, 256) : kRedBlocks, 256, 0, stream>>>(lev[l].Q, lev[l].Qf, N);
+        launches++;
+    }
     INCRMT_CKL("k_cast_stencil");
     int r = tail_pack<float>();
     if (r) return r;
@@ -1397,19 +1271,19 @@ int Multigrid::cycle64(int l, const double *b0, double *z0) {
     if (l == 0 && sys == INCRMT_SYS_MAC) {
         auto op = mac64();
         if ((r = smooth(op, z, tiles ? L.z2 : nullptr, b, L.m, L.n, kNu1, stream, launches, &cur, pf, bpu))) return r;
-        restrict_launch(tiles, op, stream, cur, b, L.m, L.n, px, py, L.kx, L.ky, C.m, C.n, C.b, C.z, L.P);
+        restrict_launch(tiles, op, stream, cur, b, px, py, L, C, C.b, C.z, L.Q);
     } else if (l == 0) {
         auto op = fem64();
         if ((r = smooth(op, z, tiles ? L.z2 : nullptr, b, L.m, L.n, kNu1, stream, launches, &cur, pf, bpu))) return r;
-        restrict_launch(tiles, op, stream, cur, b, L.m, L.n, px, py, L.kx, L.ky, C.m, C.n, C.b, C.z, L.P);
+        restrict_launch(tiles, op, stream, cur, b, px, py, L, C, C.b, C.z, L.Q);
     } else {
         if ((r = smooth(g, z, tiles ? L.z2 : nullptr, b, L.m, L.n, kNu1, stream, launches, &cur))) return r;
-        restrict_launch(tiles, g, stream, cur, b, L.m, L.n, px, py, L.kx, L.ky, C.m, C.n, C.b, C.z, L.P);
+        restrict_launch(tiles, g, stream, cur, b, px, py, L, C, C.b, C.z, L.Q);
     }
     launches++;
     INCRMT_CKL("k_restrict");
     if ((r = cycle64(l + 1, b0, z0))) return r;
-    k_prolong<<<grid2(L.m, L.n), kBlk2, 0, stream>>>(cur, L.m, L.n, px, py, L.kx, L.ky, static_cast<const double *>(C.z), C.m, C.n, L.P);
+    prolong_launch<double>(stream, cur, px, py, L, C, C.z, L.Q);
     launches++;
     INCRMT_CKL("k_prolong");
     double *alt = !tiles ? nullptr : cur == z ? L.z2 : z, *out = cur;
@@ -1483,19 +1357,19 @@ int Multigrid::cycle32(int l) {
     if (l == 0 && sys == INCRMT_SYS_MAC) {
         auto op = mac32();
         if ((r = smooth(op, z, tiles ? L.zf2 : nullptr, b, L.m, L.n, kNu1, stream, launches, &cur, pf, bpu))) return r;
-        restrict_launch(tiles, op, stream, static_cast<const float *>(cur), b, L.m, L.n, px, py, L.kx, L.ky, C.m, C.n, C.bf, C.zf, L.P);
+        restrict_launch(tiles, op, stream, static_cast<const float *>(cur), b, px, py, L, C, C.bf, C.zf, L.Qf);
     } else if (l == 0) {
         auto op = fem32();
         if ((r = smooth(op, z, tiles ? L.zf2 : nullptr, b, L.m, L.n, kNu1, stream, launches, &cur, pf, bpu))) return r;
-        restrict_launch(tiles, op, stream, static_cast<const float *>(cur), b, L.m, L.n, px, py, L.kx, L.ky, C.m, C.n, C.bf, C.zf, L.P);
+        restrict_launch(tiles, op, stream, static_cast<const float *>(cur), b, px, py, L, C, C.bf, C.zf, L.Qf);
     } else {
         if ((r = smooth(g, z, tiles ? L.zf2 : nullptr, b, L.m, L.n, kNu1, stream, launches, &cur))) return r;
-        restrict_launch(tiles, g, stream, static_cast<const float *>(cur), b, L.m, L.n, px, py, L.kx, L.ky, C.m, C.n, C.bf, C.zf, L.P);
+        restrict_launch(tiles, g, stream, static_cast<const float *>(cur), b, px, py, L, C, C.bf, C.zf, L.Qf);
     }
     launches++;
     INCRMT_CKL("k_restrict");
     if ((r = cycle32(l + 1))) return r;
-    k_prolong<<<grid2(L.m, L.n), kBlk2, 0, stream>>>(cur, L.m, L.n, px, py, L.kx, L.ky, static_cast<const float *>(C.zf), C.m, C.n, L.P);
+    prolong_launch<float>(stream, cur, px, py, L, C, C.zf, L.Qf);
     launches++;
     INCRMT_CKL("k_prolong");
     float *alt = !tiles ? nullptr : cur == z ? L.zf2 : z, *out = cur;

@@ -34,6 +34,12 @@ struct MgLevel {
     double *z2 = nullptr;  // second FP64 iterate buffer of the tile smoothers (all levels)
     double *P = nullptr;   // prolongation to the next level: four weights per unknown (all but the last)
     float *zf2 = nullptr;  // and the FP32 one
+    double *Q = nullptr;   // P's weights as planes over the cells (mg_transfer.cuh), and in FP32
+    float *Qf = nullptr;
+    /** Elements of the planes. */
+    long planes() const {
+        return (kx && ky ? 8L : 2L) * (kx ? (m + 1) / 2 : m) * (ky ? (n + 1) / 2 : n);
+    }
     double *pk = nullptr;  // stencils and transfer weights packed for the tail kernel (its levels)
     float *pkf = nullptr;
 };
