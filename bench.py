@@ -711,7 +711,7 @@ def run_ours_sim(args, ws, rank, local, dist):
                    "sample": f"unavailable: {e}"}
     sm_ms, sm_bytes, sm_launch = a["smoother"]
     roof = _roofline(f"{args.workload}_smooth", sm_ms, sm_bytes, sm_launch,
-                     "k_smooth_stream / k_smooth_tile on the fine level of the MAC and FEM projections "
+                     "k_smooth_cells on the fine level of the MAC and FEM projections "
                      "(two Gauss-Seidel sweeps per launch)",
                      "updated unknowns x 2 sweeps x (3+c) x w; c=2 MAC, 1 FEM")
     if roof is not None:
@@ -987,7 +987,7 @@ def run_ours(args, ws, rank, local, dist):
                    "krylov": bool(args.krylov)},
         "vcycles_per_projection": float(np.mean(vcs)),
         "roofline": _roofline("mac4096_smooth", kms, kbytes, klaunch,
-                              "k_smooth_stream (fine-level Gauss-Seidel, two sweeps per launch)",
+                              "k_smooth_cells (fine-level Gauss-Seidel, two sweeps per launch)",
                               "updated unknowns x 2 sweeps x (3+c) x w, c=2 (MAC)"),
         "cpu_baseline": cpu,
         "e2e": {"value": e2e, "unit": "steps/s",

@@ -3,7 +3,7 @@
 #include <cstring>
 #include <type_traits>
 #include "mg.cuh"
-#include "mg_stream.cuh"
+#include "mg_cells.cuh"
 #include "mg_tail.cuh"
 
 namespace incrmt {
@@ -299,139 +299,6 @@ __global__ void k_smooth(Op op, T *z, const T *b, int m, int n, int pi, int pj) 
 __device__ __forceinline__ int wrap_index(int i, int m) {
     i %= m;
     return i < 0 ? i + m : i;
-}
-
-/** Tile-fused Gauss-Seidel: SWEEPS complete four-colour sweeps in one launch.
- * The block stages its TW x TH tile of the iterate zin plus a halo of
- * 4*SWEEPS cells in shared memory and runs the colour phases there, phase p
- * updating the tile grown by 4*SWEEPS-1-p cells, so that every value a later
- * phase reads is already final; the tile is then written to zout. zin is not
- * written during the launch, so every block stages the values from before the
- * sweeps and each point sees exactly the neighbour values of the
- * one-launch-per-colour schedule: the result is identical to it. In a
- * periodic direction (even size) the halo holds periodic images, updated like
- * the points they copy (the colouring is consistent across the seam).
- * Coefficients and the right-hand side are read from global memory (L1/L2). */
-template <class Op, class T, int SWEEPS, int TW, int TH>
-__global__ void __launch_bounds__(256) k_smooth_tile(Op op, const T *zin, T *zout, const T *b, int m, int n) {
-    constexpr int H = 4 * SWEEPS, LW = TW + 2 * H, LH = TH + 2 * H;
-    __shared__ T zs[LW * LH];
-    const int x0 = blockIdx.x * TW, y0 = blockIdx.y * TH;
-    const int gx0 = x0 - H, gy0 = y0 - H;
-    const bool px = op.px, py = op.py;
-    for (int t = threadIdx.x; t < LW * LH; t += blockDim.x) {
-        int i = gx0 + t % LW, j = gy0 + t / LW;
-        if (px) i = wrap_index(i, m);
-        if (py) j = wrap_index(j, n);
-        if (i >= 0 && i < m && j >= 0 && j < n) zs[t] = zin[i + static_cast<long>(m) * j];
-    }
-    __syncthreads();
-    const int pis[4] = {0, 1, 1, 0}, pjs[4] = {0, 1, 0, 1};
-    constexpr int P = 4 * SWEEPS;
-#pragma unroll 1
-    for (int p = 0; p < P; p++) {
-        const int e = P - 1 - p, c = p & 3;
-        int ilo = x0 - e, ihi = x0 + TW - 1 + e, jlo = y0 - e, jhi = y0 + TH - 1 + e;
-        if (!px) {
-            if (ilo < 0) ilo = 0;
-            if (ihi > m - 1) ihi = m - 1;
-        }
-        if (!py) {
-            if (jlo < 0) jlo = 0;
-            if (jhi > n - 1) jhi = n - 1;
-        }
-        // first index of the colour's parity at or above the low bound
-        const int i0 = ilo + ((ilo & 1) != pis[c]), j0 = jlo + ((jlo & 1) != pjs[c]);
-        const int ni = i0 <= ihi ? (ihi - i0) / 2 + 1 : 0, nj = j0 <= jhi ? (jhi - j0) / 2 + 1 : 0;
-        for (int t = threadIdx.x; t < ni * nj; t += blockDim.x) {
-            const int i = i0 + 2 * (t % ni), j = j0 + 2 * (t / ni);
-            const int lz = (i - gx0) + LW * (j - gy0);
-            const int ir = px ? wrap_index(i, m) : i, jr = py ? wrap_index(j, n) : j;
-            zs[lz] = gs_update_s(op, ir, jr, zs, lz, LW, b[ir + static_cast<long>(m) * jr]);
-        }
-        __syncthreads();
-    }
-    for (int t = threadIdx.x; t < TW * TH; t += blockDim.x) {
-        const int i = x0 + t % TW, j = y0 + t / TW;
-        if (i < m && j < n) zout[i + static_cast<long>(m) * j] = zs[(i - gx0) + LW * (j - gy0)];
-    }
-}
-
-/** k_smooth_tile for the Galerkin levels' nine-point stencils with every
- * input staged up front: the nine coefficients and the right-hand side of the
- * whole halo region go to shared memory with the iterate before the first
- * phase, so the colour phases run on shared memory alone instead of waiting
- * on L2 for the coefficients in each of them (the small coarse levels are
- * latency-bound). The arithmetic, and so the result, is that of
- * k_smooth_tile. Dynamic shared memory: (11 * LW * LH) elements. */
-template <class T, int SWEEPS, int TW, int TH>
-__global__ void __launch_bounds__(256) k_smooth_tile_gen(GenOp<T> op, const T *zin, T *zout, const T *b, int m,
-                                                         int n) {
-    constexpr int H = 4 * SWEEPS, LW = TW + 2 * H, LH = TH + 2 * H, LA = LW * LH;
-    extern __shared__ __align__(16) unsigned char gen_smem[];
-    T *zs = reinterpret_cast<T *>(gen_smem);
-    T *bs = zs + LA;
-    T *cs = bs + LA;  // coefficient k of local point t at cs[k * LA + t]
-    const int x0 = blockIdx.x * TW, y0 = blockIdx.y * TH;
-    const int gx0 = x0 - H, gy0 = y0 - H;
-    const bool px = op.px, py = op.py;
-    const long N = op.N;
-    for (int t = threadIdx.x; t < LA; t += blockDim.x) {
-        int i = gx0 + t % LW, j = gy0 + t / LW;
-        if (px) i = wrap_index(i, m);
-        if (py) j = wrap_index(j, n);
-        if (i >= 0 && i < m && j >= 0 && j < n) {
-            const long ij = i + static_cast<long>(m) * j;
-            zs[t] = zin[ij];
-            bs[t] = b[ij];
-            const long q = op.at(i, j);
-#pragma unroll
-            for (int k = 0; k < 9; k++) cs[k * LA + t] = op.st[k * N + q];
-        }
-    }
-    __syncthreads();
-    const int pis[4] = {0, 1, 1, 0}, pjs[4] = {0, 1, 0, 1};
-    constexpr int P = 4 * SWEEPS;
-#pragma unroll 1
-    for (int p = 0; p < P; p++) {
-        const int e = P - 1 - p, c = p & 3;
-        int ilo = x0 - e, ihi = x0 + TW - 1 + e, jlo = y0 - e, jhi = y0 + TH - 1 + e;
-        if (!px) {
-            if (ilo < 0) ilo = 0;
-            if (ihi > m - 1) ihi = m - 1;
-        }
-        if (!py) {
-            if (jlo < 0) jlo = 0;
-            if (jhi > n - 1) jhi = n - 1;
-        }
-        const int i0 = ilo + ((ilo & 1) != pis[c]), j0 = jlo + ((jlo & 1) != pjs[c]);
-        const int ni = i0 <= ihi ? (ihi - i0) / 2 + 1 : 0, nj = j0 <= jhi ? (jhi - j0) / 2 + 1 : 0;
-        for (int t = threadIdx.x; t < ni * nj; t += blockDim.x) {
-            const int i = i0 + 2 * (t % ni), j = j0 + 2 * (t / ni);
-            const int lz = (i - gx0) + LW * (j - gy0);
-            const int ir = px ? wrap_index(i, m) : i, jr = py ? wrap_index(j, n) : j;
-            // gs_update_s of GenOp with the coefficients read from shared
-            // memory (in single precision entry 4 is the row sum and the
-            // neighbours enter centred)
-            const bool l = px || ir > 0, r = px || ir < m - 1, d = py || jr > 0, u = py || jr < n - 1;
-            const T zc = sizeof(T) == 8 ? T(0) : zs[lz];
-            T diag = cs[4 * LA + lz];
-            const T rs = diag;  // the row sum in single precision
-            const T s = GenOp<T>::template gen_sum<sizeof(T) == 4>(l, r, d, u, cs + lz, LA, zs + lz, 1, LW, zc, diag);
-            zs[lz] = gs_value(bs[lz], s, diag, zc, rs);
-        }
-        __syncthreads();
-    }
-    for (int t = threadIdx.x; t < TW * TH; t += blockDim.x) {
-        const int i = x0 + t % TW, j = y0 + t / TW;
-        if (i < m && j < n) zout[i + static_cast<long>(m) * j] = zs[(i - gx0) + LW * (j - gy0)];
-    }
-}
-
-/** Shared memory of k_smooth_tile_gen<T, SWEEPS, TW, TH>. */
-template <class T, int SWEEPS = 2, int TW = 16, int TH = 16>
-constexpr int gen_tile_smem() {
-    return 11 * (TW + 8 * SWEEPS) * (TH + 8 * SWEEPS) * static_cast<int>(sizeof(T));
 }
 
 /** Coarse right-hand side b_c = P^T (b - A z), the fine residual formed on
@@ -808,18 +675,6 @@ constexpr int kRedBlocks = 4 * kB200SMs;  // reduction grid: 4 x 148 blocks of 2
 inline dim3 grid2(int m, int n) { return dim3(cdiv(m, 32), cdiv(n, 8)); }
 const dim3 kBlk2(32, 8);
 
-/** Which systems' large levels run as a pipeline along y, and from how many
- * unknowns on (mg_stream.cuh has both sides' times): the five-point one in
- * both precisions, the FEM system in single. */
-template <class Op, class T>
-constexpr bool kStreams = false;
-template <class T>
-constexpr bool kStreams<MacOp<T>, T> = true;
-template <>
-constexpr bool kStreams<FemOp<float>, float> = true;
-template <class Op>
-constexpr long kStreamMin = Op::kFivePoint ? 512L * 512 : 1500L * 1500;
-
 /** The attributes a launch of k_tail needs. */
 template <class T, bool SEQ>
 cudaError_t set_tail_attr() {
@@ -840,30 +695,11 @@ int smooth(Op op, T *z, T *zalt, const T *b, int m, int n, int sweeps, cudaStrea
            Multigrid *prof = nullptr, double bytes_per_unit = 0) {
     *res = z;
     if (sweeps == 2 && zalt && (!op.px || m % 2 == 0) && (!op.py || n % 2 == 0)) {
-        // Two sweeps per launch with shared-memory tiles (identical results);
-        // the largest tile that still gives every SM work, else the smallest.
-        const dim3 b64(cdiv(m, 64), cdiv(n, 32)), b32(cdiv(m, 32), cdiv(n, 16)), b16(cdiv(m, 16), cdiv(n, 16));
         if (prof) { int r = prof->prof_begin(static_cast<double>(m) * n * 2 * bytes_per_unit); if (r) return r; }
-        bool done = false;
-        if constexpr (kStreams<Op, T>) {
-            if (static_cast<long>(m) * n >= kStreamMin<Op>) {
-                const StreamGrid<Op, T> sg(m, n);
-                k_smooth_stream<Op, T><<<sg.grid, 256, stream_elems<Op>() * sizeof(T), s>>>(op, z, zalt, b, m, n, sg.chunk);
-                done = true;
-            }
-        }
-        if (done) {
-        } else if (static_cast<int>(b64.x * b64.y) >= 2 * kB200SMs)
-            k_smooth_tile<Op, T, 2, 64, 32><<<b64, 256, 0, s>>>(op, z, zalt, b, m, n);
-        else if (static_cast<int>(b32.x * b32.y) >= kB200SMs)
-            k_smooth_tile<Op, T, 2, 32, 16><<<b32, 256, 0, s>>>(op, z, zalt, b, m, n);
-        else if constexpr (std::is_same<Op, GenOp<T>>::value)
-            k_smooth_tile_gen<T, 2, 16, 16><<<b16, 256, gen_tile_smem<T>(), s>>>(op, z, zalt, b, m, n);
-        else
-            k_smooth_tile<Op, T, 2, 16, 16><<<b16, 256, 0, s>>>(op, z, zalt, b, m, n);
+        smooth_cells(op, z, zalt, b, m, n, s);
         nl++;
         if (prof) { int r = prof->prof_end(); if (r) return r; }
-        INCRMT_CKL("k_smooth_tile");
+        INCRMT_CKL("k_smooth_cells");
         *res = zalt;
         return INCRMT_OK;
     }
@@ -1024,17 +860,10 @@ int Multigrid::build_hierarchy() {
         INCRMT_CK(cudaFuncSetAttribute(k_coarse_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(sizeof(double) * (2 * kDirectMax * kDirectMax + kDirectMax))));
     }
-    INCRMT_CK((set_stream_attr<MacOp<double>, double>()));
-    INCRMT_CK((set_stream_attr<MacOp<float>, float>()));
-    INCRMT_CK((set_stream_attr<FemOp<float>, float>()));
     INCRMT_CK((set_tail_attr<double, false>()));
     INCRMT_CK((set_tail_attr<double, true>()));
     INCRMT_CK((set_tail_attr<float, false>()));
     INCRMT_CK((set_tail_attr<float, true>()));
-    INCRMT_CK(cudaFuncSetAttribute(k_smooth_tile_gen<double, 2, 16, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   gen_tile_smem<double>()));
-    INCRMT_CK(cudaFuncSetAttribute(k_smooth_tile_gen<float, 2, 16, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   gen_tile_smem<float>()));
     const int gal_smem = static_cast<int>(galerkin_tile_smem(true, true));
     INCRMT_CK(set_galerkin_attr<MacOp<double>>(gal_smem));
     INCRMT_CK(set_galerkin_attr<FemOp<double>>(gal_smem));

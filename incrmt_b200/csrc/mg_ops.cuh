@@ -77,7 +77,7 @@ struct MacOp {
         const T el = ex[j * (m + 1) + i], er = ex[j * (m + 1) + i + 1];
         const T ed = ey[j * m + i], eu = ey[(j + 1) * m + i];
         const bool l = px || i > 0, r = px || i < m - 1, d = py || j > 0, u = py || j < n - 1;
-        // neighbour indices wrap, so every load is in range (see GenOp::gen_sum)
+        // neighbour indices wrap, so every load is in range (see GenOp::gen_terms)
         const T zl = z[i > 0 ? ij - 1 : ij + m - 1], zr = z[i < m - 1 ? ij + 1 : ij + 1 - m];
         const T zd = z[j > 0 ? ij - m : ij + m * (n - 1)], zu = z[j < n - 1 ? ij + m : ij - m * (n - 1)];
         diag = diag_of(i, l, r, d, u, el, er, ed, eu);
@@ -109,26 +109,6 @@ struct MacOp {
     __device__ __forceinline__ T rowsum(int i, int j) const {
         if (!zpr || px || i != m - 1) return T(0);
         return -2 * xxsp * ex[j * (m + 1) + i + 1];
-    }
-
-    /** offdiag with the iterate in a shared-memory tile (lz: local index of
-     * (i,j), ldz: tile row stride). The tile holds the neighbours at lz+-1,
-     * lz+-ldz, across a periodic edge too (as periodic images). */
-    template <bool CEN = false>
-    __device__ __forceinline__ T offdiag_s(int i, int j, const T *zs, int lz, int ldz, T &diag) const {
-        return offdiag_v<CEN>(i, j, ex[j * (m + 1) + i], ex[j * (m + 1) + i + 1], ey[j * m + i], ey[(j + 1) * m + i],
-                              zs, lz, ldz, diag);
-    }
-
-    /** offdiag_s with the four edge coefficients of (i,j) given (left, right,
-     * below, above), e.g. staged in shared memory. */
-    template <bool CEN = false>
-    __device__ __forceinline__ T offdiag_v(int i, int j, T el, T er, T ed, T eu, const T *zs, int lz, int ldz,
-                                           T &diag) const {
-        const bool l = px || i > 0, r = px || i < m - 1, d = py || j > 0, u = py || j < n - 1;
-        const T zc = CEN ? zs[lz] : T(0);
-        diag = diag_of(i, l, r, d, u, el, er, ed, eu);
-        return mac_terms<CEN>(l, r, d, u, el, er, ed, eu, zs[lz - 1], zs[lz + 1], zs[lz - ldz], zs[lz + ldz], zc);
     }
 
     __device__ __forceinline__ void coef9(int i, int j, T a[9]) const {
@@ -195,16 +175,9 @@ struct FemOp {
         a[5] = r ? ((d ? cdr : T(0)) + (u ? cur : T(0))) * hex : T(0);
     }
 
-    template <bool CEN = false>
-    __device__ __forceinline__ T offdiag_s(int i, int j, const T *zs, int lz, int ldz, T &diag) const {
-        const int ij = i + m * j;
-        if (i > 0 && i < m - 1 && j > 0 && j < n - 1)
-            return offdiag_int<CEN>(c[ij], c[ij + 1], c[ij + m], c[ij + m + 1], zs, lz, ldz, diag);
-        return offdiag_edge<CEN>(i, j, zs, lz, ldz, diag);
-    }
-
-    /** offdiag_s at an interior node, the four cell values around it given
-     * (below-left, below-right, above-left, above-right). */
+    /** The off-diagonal sum at an interior node, the iterate at zs[lz] with row
+     * stride ldz and the four cell values around the node given (below-left,
+     * below-right, above-left, above-right). */
     template <bool CEN = false>
     __device__ __forceinline__ T offdiag_int(T cdl, T cdr, T cul, T cur, const T *zs, int lz, int ldz,
                                              T &diag) const {
@@ -219,15 +192,7 @@ struct FemOp {
         return fma_rn(cdr, cell(1, -ldz), fma_rn(cur, cell(1, ldz), fma_rn(cdl, cell(-1, -ldz), mul_rn(cul, cell(-1, ldz)))));
     }
 
-    /** offdiag_s at a node on an edge of the grid (the cells from c). */
-    template <bool CEN = false>
-    __device__ __forceinline__ T offdiag_edge(int i, int j, const T *zs, int lz, int ldz, T &diag) const {
-        T cdl, cdr, cul, cur;
-        cells(i, j, cdl, cdr, cul, cur);
-        return offdiag_cells<CEN>(i, j, cdl, cdr, cul, cur, zs, lz, ldz, diag);
-    }
-
-    /** offdiag_edge, the four cell values around the node given. */
+    /** offdiag_int for a node on an edge of the grid. */
     template <bool CEN = false>
     __device__ __forceinline__ T offdiag_cells(int i, int j, T cdl, T cdr, T cul, T cur, const T *zs, int lz, int ldz,
                                                T &diag) const {
@@ -323,40 +288,14 @@ struct GenOp {
         for (int k = 0; k < 9; k++) a[k] = st[k * N + q];
     }
 
-    /** With CEN (the single-precision stencils, whose entry 4 holds the row
-     * sum, see galerkin_all), the centred off-diagonal sum; diag is then the
-     * row sum minus the off-diagonal entries. */
-    template <bool CEN = false>
-    __device__ __forceinline__ T offdiag_s(int i, int j, const T *zs, int lz, int ldz, T &diag) const {
-        const long q = at(i, j);
-        const T zc = CEN ? zs[lz] : T(0);
-        diag = st[4 * N + q];
-        return gen_sum<CEN>(px || i > 0, px || i < m - 1, py || j > 0, py || j < n - 1, st + q, N, zs + lz, 1, ldz,
-                            zc, diag);
-    }
-
-    /** The off-diagonal sum over the entries c[k*ldc] (k = 0..8, in the
-     * order dl,dc,dr,cl,cr,ul,uc,ur) of a point whose iterate is w[0],
-     * neighbours at w[+-dx], w[+-dy]; diag holds entry 4 on entry and, with
-     * CEN, the row sum minus the off-diagonal entries on return. Shared by
-     * every nine-point smoother so that all of them round alike. */
-    template <bool CEN, class C>
-    static __device__ __forceinline__ T gen_sum(bool l, bool r, bool d, bool u, const C *c, long ldc, const T *w,
-                                                int dx, int dy, T zc, T &diag) {
-        // Every entry and neighbour is read unconditionally (the point's own
-        // entries, and neighbours inside the caller's array: a shared-memory
-        // tile with a halo, or a wrapped global index), so that all eighteen
-        // loads can be in flight at once; the terms outside the grid are then
-        // skipped by selection, which leaves the sum as the branches would.
-        const T k0 = c[0], k1 = c[ldc], k2 = c[2 * ldc], k3 = c[3 * ldc], k5 = c[5 * ldc], k6 = c[6 * ldc],
-                k7 = c[7 * ldc], k8 = c[8 * ldc];
-        const T z0 = w[-dy - dx], z1 = w[-dy], z2 = w[-dy + dx], z3 = w[-dx], z5 = w[dx], z6 = w[dy - dx],
-                z7 = w[dy], z8 = w[dy + dx];
-        return gen_terms<CEN>(l, r, d, u, k0, k1, k2, k3, k5, k6, k7, k8, z0, z1, z2, z3, z5, z6, z7, z8, zc, diag);
-    }
-
     /** The off-diagonal sum from the eight entries and neighbour values
-     * (order dl,dc,dr,cl,cr,ul,uc,ur), terms outside the grid skipped. */
+     * (order dl,dc,dr,cl,cr,ul,uc,ur). diag holds entry 4 on entry and, with
+     * CEN (the single-precision stencils, whose entry 4 is the row sum), the row
+     * sum minus the off-diagonal entries on return. The caller reads every entry
+     * and neighbour, so that all the loads can be in flight at once; the terms
+     * outside the grid are then skipped by selection, which leaves the sum as
+     * branches would. Shared by every nine-point smoother so that all of them
+     * round alike. */
     template <bool CEN>
     static __device__ __forceinline__ T gen_terms(bool l, bool r, bool d, bool u, T k0, T k1, T k2, T k3, T k5, T k6,
                                                   T k7, T k8, T z0, T z1, T z2, T z3, T z5, T z6, T z7, T z8, T zc,
@@ -418,20 +357,6 @@ __device__ __forceinline__ T gs_update(const Op &op, int i, int j, const T *z, T
     } else {
         const T zc = z[i + static_cast<long>(op.m) * j];
         const T off = op.template offdiag<true>(i, j, z, diag, zc);
-        return gs_value(b, off, diag, zc, op.rowsum(i, j));
-    }
-}
-
-/** gs_update with the iterate in a shared-memory tile. */
-template <class Op, class T>
-__device__ __forceinline__ T gs_update_s(const Op &op, int i, int j, const T *zs, int lz, int ldz, T b) {
-    T diag;
-    if constexpr (sizeof(T) == 8) {
-        const T off = op.offdiag_s(i, j, zs, lz, ldz, diag);
-        return gs_value(b, off, diag, T(0), T(0));
-    } else {
-        const T zc = zs[lz];
-        const T off = op.template offdiag_s<true>(i, j, zs, lz, ldz, diag);
         return gs_value(b, off, diag, zc, op.rowsum(i, j));
     }
 }

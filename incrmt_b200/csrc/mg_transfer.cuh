@@ -17,9 +17,8 @@
 namespace incrmt {
 namespace {
 
-/** Cells of a level, and its weight planes. */
+/** Cells of a level along an axis. */
 __host__ __device__ __forceinline__ int cells_of(int m, bool k) { return k ? (m + 1) >> 1 : m; }
-__host__ __device__ __forceinline__ int planes_of(bool kx, bool ky) { return kx && ky ? 8 : 2; }
 
 constexpr int kPX = 32, kPY = 8;  // cells of a block of k_build_p
 

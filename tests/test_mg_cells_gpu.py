@@ -1,7 +1,8 @@
-"""The fine levels' pipelined smoothing (k_smooth_stream) against one launch per
-colour, bit for bit: grids just above its size threshold, odd sizes, strips
-whose last columns are one cell or a full strip, chunks of one row, and seams
-in either direction with densities that do not match across them."""
+"""The smoother by cells (k_smooth_cells), with the transfers and Galerkin
+products by tiles, against one launch per colour and per point, bit for bit:
+sizes around a tile's edges and around the rules that choose its height, odd
+sizes, grids of many or few tiles, arrays that cannot be read by pairs, and
+seams in either direction with densities that do not match across them."""
 import numpy as np
 import pytest
 
@@ -17,13 +18,24 @@ CASES = [
     (0, 17, 16384, False, False, False, False),    # one strip, many chunks
     (0, 600, 512, True, True, False, False),
     (0, 1536, 320, False, True, True, True),
+    (0, 112, 96, False, False, False, True),       # two MAC tiles by four
+    (0, 114, 98, False, False, True, True),        # one cell more
+    (0, 111, 95, False, False, False, True),
+    (0, 128, 130, True, True, False, True),
+    (1, 107, 95, False, False, False, True),       # 108 x 96 nodes: two tiles of 27 cells, six of 8
+    (1, 108, 96, False, False, True, True),
+    (1, 160, 160, True, True, False, True),
+    (1, 511, 289, False, False, True, True),       # either height, double
+    (1, 760, 900, False, False, False, True),      # either height, single
+    (1, 1100, 1024, False, True, False, True),
     (1, 1601, 1499, False, False, False, True),
     (1, 1536, 1600, False, True, True, True),
 ]
 
 
 @pytest.mark.parametrize("sys_,m,n,xp,yp,zpr,mixed", CASES)
-def test_stream_identical_to_colour_launches(gpu, sys_, m, n, xp, yp, zpr, mixed):
+@pytest.mark.parametrize("shift", [0, 1])
+def test_cells_identical_to_colour_launches(gpu, sys_, m, n, xp, yp, zpr, mixed, shift):
     import torch
     from incrmt_b200 import capi
     s = capi.MGSolver(sys_, m, n, bx=-1 + 2 * m / max(m, n), by=-1 + 2 * n / max(m, n), x_prd=xp, y_prd=yp, zpr=zpr)
@@ -33,7 +45,8 @@ def test_stream_identical_to_colour_launches(gpu, sys_, m, n, xp, yp, zpr, mixed
     b = rng.standard_normal(N)
     b -= b.mean()
     z0 = rng.standard_normal(N)
-    bd = torch.tensor(b, device="cuda")
+    bd = torch.zeros(N + 1, dtype=torch.float64, device="cuda")[shift:shift + N]  # shift 1: rows start off a pair
+    bd.copy_(torch.tensor(b))
     out = {}
     for tiles in (True, False):
         s.set_tiles(tiles)
