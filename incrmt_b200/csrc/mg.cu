@@ -452,24 +452,116 @@ __global__ void k_coarse_inverse(const double *st, int m, int n, int px, int py,
     }
 }
 
-/** FP64 residual r = b - A z, optionally stored in FP32, with per-block sums
- * of r^2 in partial[blockIdx.x]. Each block takes every gridDim.x-th row,
- * its threads the row's unknowns (coalesced, no index division). */
+/** The total of the blocks' sums acc (256 threads each), in the order of the
+ * blocks whichever finishes last: that one adds the partials up, so the sum
+ * needs no launch of its own. True in its first thread, with the total in acc.
+ * *ticket is zero before and after. */
+__device__ __forceinline__ bool grid_sum_256(double &acc, double *partial, unsigned *ticket) {
+    __shared__ bool last;
+    acc = block_sum_256(acc);
+    if (threadIdx.x == 0) {
+        partial[blockIdx.x] = acc;
+        __threadfence();
+        last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return false;
+    __threadfence();
+    acc = 0;
+    for (int q = threadIdx.x; q < gridDim.x; q += 256) acc += __ldcg(partial + q);
+    acc = block_sum_256(acc);
+    return threadIdx.x == 0;
+}
+
+/** What the residual at a point reads; load() takes everything without a
+ * branch, so that the loads of several points are in flight together. */
 template <class Op>
-__global__ void k_resnorm(Op op, const double *z, const double *b, int m, int n, float *rf,
-                          double *partial) {
+struct ResPoint;
+template <>
+struct ResPoint<MacOp<double>> {
+    double off, diag, zc, b;
+    __device__ __forceinline__ void load(const MacOp<double> &op, const double *__restrict__ z, const double *__restrict__ rhs, int i,
+                                         int j) {
+        const int q = i + op.m * j;
+        off = op.offdiag(i, j, z, diag);
+        zc = z[q];
+        b = rhs[q];
+    }
+    __device__ __forceinline__ double residual(const MacOp<double> &, int, int) const { return fma_rn(-diag, zc, sub_rn(b, off)); }
+};
+template <>
+struct ResPoint<FemOp<double>> {
+    double w[9], cdl, cdr, cul, cur, b;
+    __device__ __forceinline__ void load(const FemOp<double> &op, const double *__restrict__ z, const double *__restrict__ rhs, int i,
+                                         int j) {
+        const int m = op.m, n = op.n, q = i + m * j;
+        const int il = i > 0 ? -1 : m - 1, ir = i < m - 1 ? 1 : 1 - m;
+        const int jd = j > 0 ? -m : m * (n - 1), ju = j < n - 1 ? m : -m * (n - 1);
+        const double *v = z + q;
+        w[0] = v[jd + il]; w[1] = v[jd]; w[2] = v[jd + ir];
+        w[3] = v[il];      w[4] = v[0];  w[5] = v[ir];
+        w[6] = v[ju + il]; w[7] = v[ju]; w[8] = v[ju + ir];
+        op.cells(i, j, cdl, cdr, cul, cur);
+        b = rhs[q];
+    }
+    __device__ __forceinline__ double residual(const FemOp<double> &op, int i, int j) const {
+        double diag, off;
+        if (i > 0 && i < op.m - 1 && j > 0 && j < op.n - 1) off = op.offdiag_int(cdl, cdr, cul, cur, w, 4, 3, diag);
+        else off = op.offdiag_cells(i, j, cdl, cdr, cul, cur, w, 4, 3, diag);
+        return fma_rn(-diag, w[4], sub_rn(b, off));
+    }
+};
+
+/** Whether the V-cycles go on after one that left the squared residual rn2, by
+ * the tests that follow them on the host: solved, not finite, no longer
+ * halving in mixed precision, or at the limit. */
+__device__ __forceinline__ bool loop_goes_on(MgLoop *p, double rn2, double *host) {
+    const double rn = sqrt(rn2), prev = p->prev;
+    const int k = ++p->k;
+    host[0] = rn2;
+    host[1] = k;
+    host[2] = prev;
+    p->prev = rn;
+    return isfinite(rn) && rn > p->tol && !(p->mixed && rn > kMixedContraction * prev) && k < p->maxc;
+}
+
+__global__ void k_loop_begin(MgLoop *p, double tol, double prev, int k, int maxc, int mixed) {
+    *p = MgLoop{tol, prev, k, maxc, mixed};
+}
+
+/** FP64 residual r = b - A z, optionally stored in FP32, and the sum of r^2 in
+ * the host's host[0]. Each block takes every gridDim.x-th row, its threads the
+ * row's unknowns (coalesced, no index division). Bound by memory once the loads
+ * of a point, or of two five-point ones, are in flight together: 4096^2 MAC 144
+ * -> 101 us (four points 107), FEM 140 -> 108 (two points spill: 187), of 82 and
+ * 61 us for the bytes. The total and its way to the host are this launch's too
+ * (small grids: 2.1 us, 1.9 for the sum and 3.3 for the copy before, 4.5 now).
+ * As the end of a captured loop's body it also decides whether that runs again. */
+template <class Op>
+__global__ void __launch_bounds__(256, 4) k_resnorm(Op op, const double *__restrict__ z, const double *__restrict__ b, int m, int n,
+                                                    float *__restrict__ rf, double *partial, unsigned *ticket, double *host,
+                                                    MgLoop *loop, cudaGraphConditionalHandle body) {
+    constexpr int U = Op::kFivePoint ? 2 : 1;
     double acc = 0;
     for (int j = blockIdx.x; j < n; j += gridDim.x)
-        for (int i = threadIdx.x; i < m; i += blockDim.x) {
-            const long q = i + static_cast<long>(m) * j;
-            double diag;
-            const double off = op.offdiag(i, j, z, diag);
-            const double r = fma_rn(-diag, z[q], sub_rn(b[q], off));
-            if (rf) rf[q] = static_cast<float>(r);
-            acc += r * r;
+        for (int i = threadIdx.x; i < m; i += U * 256) {
+            ResPoint<Op> p[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) p[u].load(op, z, b, min(i + 256 * u, m - 1), j);
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int k = i + 256 * u;
+                if (k < m) {
+                    const double r = p[u].residual(op, k, j);
+                    if (rf) rf[k + static_cast<long>(m) * j] = static_cast<float>(r);
+                    acc += r * r;
+                }
+            }
         }
-    acc = block_sum_256(acc);
-    if (threadIdx.x == 0) partial[blockIdx.x] = acc;
+    if (grid_sum_256(acc, partial, ticket)) {
+        if (loop) cudaGraphSetConditional(body, loop_goes_on(loop, acc, host));
+        else host[0] = acc;
+    }
 }
 
 /** out = A z. */
@@ -499,14 +591,13 @@ __global__ void k_reduce(const double *partial, int nb, double *out) {
     if (threadIdx.x == 0) *out = acc;
 }
 
-/** Per-block sums of an FP32 array, accumulated in FP64. */
-__global__ void k_sum_f32(const float *a, long N, double *partial) {
+/** Sum of an FP32 array, accumulated in FP64. */
+__global__ void k_sum_f32(const float *a, long N, double *partial, unsigned *ticket, double *out) {
     double acc = 0;
     for (long q = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; q < N;
          q += static_cast<long>(gridDim.x) * blockDim.x)
         acc += static_cast<double>(a[q]);
-    acc = block_sum_256(acc);
-    if (threadIdx.x == 0) partial[blockIdx.x] = acc;
+    if (grid_sum_256(acc, partial, ticket)) *out = acc;
 }
 
 /** z += e - mean(e), the mean from the sum in *sum (a correction of a
@@ -802,7 +893,10 @@ int Multigrid::create(int sys_, int cm_, int cn_, double ax, double bx, double a
     INCRMT_CK(cudaMalloc(&bbuf, sizeof(double) * N));
     INCRMT_CK(cudaMalloc(&zbuf, sizeof(double) * N));
     INCRMT_CK(cudaMalloc(&partial, sizeof(double) * kRedBlocks));
-    INCRMT_CK(cudaMalloc(&dnorm, sizeof(double) * 4));
+    INCRMT_CK(cudaMalloc(&dnorm, sizeof(double) * 8 + sizeof(MgLoop)));
+    ticket = reinterpret_cast<unsigned *>(dnorm + 4);
+    loop = reinterpret_cast<MgLoop *>(dnorm + 8);
+    INCRMT_CK(cudaMemsetAsync(ticket, 0, sizeof(unsigned), stream));
     INCRMT_CK(cudaMallocHost(&hnorm, sizeof(double) * 4));
     return build_hierarchy();
 }
@@ -847,9 +941,9 @@ int Multigrid::build_hierarchy() {
     }
     // Prolongation weights of every level but the coarsest (k_build_p).
     for (size_t l = 0; l + 1 < lev.size(); l++) {
-        INCRMT_CK(cudaMalloc(&lev[l].P, sizeof(double) * 4 * lev[l].N));
-        INCRMT_CK(cudaMemsetAsync(lev[l].P, 0, sizeof(double) * 4 * lev[l].N, stream));
-        INCRMT_CK(cudaMalloc(&lev[l].Q, (sizeof(double) + sizeof(float)) * lev[l].planes()));
+        // the weights and, behind them, their planes in both precisions
+        INCRMT_CK(cudaMalloc(&lev[l].P, sizeof(double) * 4 * lev[l].N + (sizeof(double) + sizeof(float)) * lev[l].planes()));
+        lev[l].Q = lev[l].P + 4 * lev[l].N;
         lev[l].Qf = reinterpret_cast<float *>(lev[l].Q + lev[l].planes());
     }
     if (lev.size() > 1 && lev.back().N <= kDirectMax) {
@@ -874,7 +968,7 @@ int Multigrid::build_hierarchy() {
 void Multigrid::destroy() {
     for (auto &L : lev) {
         cudaFree(L.z); cudaFree(L.b); cudaFree(L.st); cudaFree(L.zf); cudaFree(L.bf); cudaFree(L.stf);
-        cudaFree(L.z2); cudaFree(L.zf2); cudaFree(L.P); cudaFree(L.Q);
+        cudaFree(L.z2); cudaFree(L.zf2); cudaFree(L.P);
     }
     lev.clear();
     cudaFree(ex); cudaFree(ey); cudaFree(exf); cudaFree(eyf); cudaFree(c); cudaFree(cf);
@@ -1401,12 +1495,13 @@ int Multigrid::norm2_rhs(const double *b, double *out_dev) {
     return INCRMT_OK;
 }
 
-int Multigrid::residual_norm(const double *b, const double *z, float *rf, double *out_dev) {
+int Multigrid::residual_norm(const double *b, const double *z, float *rf, const cudaGraphConditionalHandle *body) {
     const int nb = n < kRedBlocks ? n : kRedBlocks;  // blocks over the rows
-    if (sys == INCRMT_SYS_MAC) k_resnorm<<<nb, 256, 0, stream>>>(mac64(), z, b, m, n, rf, partial);
-    else k_resnorm<<<nb, 256, 0, stream>>>(fem64(), z, b, m, n, rf, partial);
-    k_reduce<<<1, 256, 0, stream>>>(partial, nb, out_dev);
-    launches += 2;
+    const cudaGraphConditionalHandle h = body ? *body : 0;
+    MgLoop *p = body ? loop : nullptr;
+    if (sys == INCRMT_SYS_MAC) k_resnorm<<<nb, 256, 0, stream>>>(mac64(), z, b, m, n, rf, partial, ticket, hnorm, p, h);
+    else k_resnorm<<<nb, 256, 0, stream>>>(fem64(), z, b, m, n, rf, partial, ticket, hnorm, p, h);
+    launches++;
     INCRMT_CKL("residual norm");
     return INCRMT_OK;
 }
@@ -1419,13 +1514,13 @@ int Multigrid::fetch_norm(double *v) {
 }
 
 /** One V-cycle (FP64, or one FP32 defect-correction step in mixed mode),
- * the FP64 residual norm of the new iterate, and its copy to hnorm[0]. */
-int Multigrid::vcycle_and_norm(int prec, const double *b, double *d_z, long N) {
+ * the FP64 residual norm of the new iterate in hnorm[0]. */
+int Multigrid::vcycle_and_norm(int prec, const double *b, double *d_z, long N, const cudaGraphConditionalHandle *body) {
     int r;
     const long long l0 = launches;
     if (prec == INCRMT_PREC_FP64) {
         if ((r = cycle64(0, b, d_z))) return r;
-        if ((r = residual_norm(b, d_z, nullptr, dnorm))) return r;
+        if ((r = residual_norm(b, d_z, nullptr, body))) return r;
     } else {
         const int nbk = cdiv(N, 256) < kRedBlocks ? cdiv(N, 256) : kRedBlocks;
         k_fill<float><<<nbk, 256, 0, stream>>>(lev[0].zf, N, 0.f);
@@ -1439,15 +1534,13 @@ int Multigrid::vcycle_and_norm(int prec, const double *b, double *d_z, long N) {
             // constants): the FP32 cycle's correction comes back with a
             // constant part thousands of times its variation on the finest
             // grids, which the iterate would accumulate; it is removed.
-            k_sum_f32<<<nbk, 256, 0, stream>>>(lev[0].zf, N, partial);
-            k_reduce<<<1, 256, 0, stream>>>(partial, nbk, dnorm + 1);
+            k_sum_f32<<<nbk, 256, 0, stream>>>(lev[0].zf, N, partial, ticket, dnorm + 1);
             k_add_f32_centred<<<nbk, 256, 0, stream>>>(d_z, lev[0].zf, N, dnorm + 1);
-            launches += 3;
+            launches += 2;
         }
         INCRMT_CKL("defect correction");
-        if ((r = residual_norm(b, d_z, lev[0].bf, dnorm))) return r;
+        if ((r = residual_norm(b, d_z, lev[0].bf, body))) return r;
     }
-    INCRMT_CK(cudaMemcpyAsync(hnorm, dnorm, sizeof(double), cudaMemcpyDeviceToHost, stream));
     graph_launches = launches - l0;
     return INCRMT_OK;
 }
@@ -1688,21 +1781,45 @@ int Multigrid::solve_device(const double *d_b, double *d_z, const incrmt_mg_opts
         }
     } else if (prec == INCRMT_PREC_MIXED) {
         if ((r = cast_levels())) return r;
-        if ((r = residual_norm(b, d_z, lev[0].bf, dnorm))) return r;
-        if ((r = fetch_norm(&rn2))) return r;
+        if ((r = residual_norm(b, d_z, lev[0].bf, nullptr))) return r;
+        INCRMT_CK(cudaStreamSynchronize(stream));
+        rn2 = hnorm[0];
         rn_prev = std::sqrt(rn2);
     }
-    // One V-cycle, its residual norm and the read-back of that norm, captured
-    // once into a CUDA graph per (precision, b, z) and replayed per cycle.
+    // V-cycles and their residual norms until one of the tests below ends them,
+    // captured once into a CUDA graph per (precision, b, z): the body of a loop
+    // that the last kernel of each cycle continues or leaves. One launch and one
+    // synchronisation per solve instead of per cycle, a round trip of about
+    // 10 us (MAC 64^2, eight cycles, 603 -> 547 us; FEM 193 x 144, thirteen, 1688
+    // -> 1531), against 0.2 ms more for the first solve with new buffers.
     const bool use_graph = !prof;
     auto capture = [&]() -> int {
         if (gexec) { cudaGraphExecDestroy(gexec); gexec = nullptr; }
         cudaGraph_t graph = nullptr;
-        INCRMT_CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-        int rc = vcycle_and_norm(cur, b, d_z, N);
-        cudaError_t ce = cudaStreamEndCapture(stream, &graph);
+        INCRMT_CK(cudaGraphCreate(&graph, 0));
+        cudaGraphConditionalHandle body;
+        cudaGraphNodeParams np = {};
+        cudaGraphNode_t node;
+        cudaError_t ce = cudaGraphConditionalHandleCreate(&body, graph, 1, cudaGraphCondAssignDefault);
+        if (ce == cudaSuccess) {
+            np.type = cudaGraphNodeTypeConditional;
+            np.conditional.handle = body;
+            np.conditional.type = cudaGraphCondTypeWhile;
+            np.conditional.size = 1;
+            ce = cudaGraphAddNode(&node, graph, nullptr, 0, &np);
+        }
+        if (ce == cudaSuccess)
+            ce = cudaStreamBeginCaptureToGraph(stream, np.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                               cudaStreamCaptureModeThreadLocal);
+        if (ce != cudaSuccess) {
+            cudaGraphDestroy(graph);
+            return cuda_status(ce, "capture", __FILE__, __LINE__);
+        }
+        int rc = vcycle_and_norm(cur, b, d_z, N, &body);
+        cudaGraph_t captured = nullptr;
+        ce = cudaStreamEndCapture(stream, &captured);
         if (rc || ce != cudaSuccess) {
-            if (ce == cudaSuccess && graph) cudaGraphDestroy(graph);
+            cudaGraphDestroy(graph);
             if (rc) return rc;
             return cuda_status(ce, "capture", __FILE__, __LINE__);
         }
@@ -1716,16 +1833,19 @@ int Multigrid::solve_device(const double *d_b, double *d_z, const incrmt_mg_opts
         return r;
     while (plain && k < maxc) {
         if (use_graph) {
+            k_loop_begin<<<1, 1, 0, stream>>>(loop, tol, rn_prev, k, maxc, cur == INCRMT_PREC_MIXED);
             INCRMT_CK(cudaGraphLaunch(gexec, stream));
-            launches += graph_launches;
             INCRMT_CK(cudaStreamSynchronize(stream));
             rn2 = hnorm[0];
+            launches += 1 + graph_launches * (static_cast<int>(hnorm[1]) - k);
+            k = static_cast<int>(hnorm[1]);
+            rn_prev = hnorm[2];
         } else {
-            if ((r = vcycle_and_norm(cur, b, d_z, N))) return r;
+            if ((r = vcycle_and_norm(cur, b, d_z, N, nullptr))) return r;
             INCRMT_CK(cudaStreamSynchronize(stream));
             rn2 = hnorm[0];
+            k++;
         }
-        k++;
         const double rn = std::sqrt(rn2);
         if (!std::isfinite(rn)) { finite = false; break; }
         if (rn <= tol) { conv = true; break; }

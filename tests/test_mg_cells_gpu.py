@@ -2,7 +2,9 @@
 products by tiles, against one launch per colour and per point, bit for bit:
 sizes around a tile's edges and around the rules that choose its height, odd
 sizes, grids of many or few tiles, arrays that cannot be read by pairs, and
-seams in either direction with densities that do not match across them."""
+seams in either direction with densities that do not match across them (periodic
+sizes that stay even down to the levels one launch holds: a larger odd periodic
+level is swept by colours that meet at its seam, in no fixed order)."""
 import numpy as np
 import pytest
 
@@ -16,12 +18,12 @@ CASES = [
     (0, 240, 1201, False, False, False, True),     # two full strips
     (0, 16384, 17, False, False, False, False),    # more strips than blocks in a wave
     (0, 17, 16384, False, False, False, False),    # one strip, many chunks
-    (0, 600, 512, True, True, False, False),
+    (0, 640, 512, True, True, False, False),
     (0, 1536, 320, False, True, True, True),
     (0, 112, 96, False, False, False, True),       # two MAC tiles by four
     (0, 114, 98, False, False, True, True),        # one cell more
     (0, 111, 95, False, False, False, True),
-    (0, 128, 130, True, True, False, True),
+    (0, 128, 160, True, True, False, True),
     (1, 107, 95, False, False, False, True),       # 108 x 96 nodes: two tiles of 27 cells, six of 8
     (1, 108, 96, False, False, True, True),
     (1, 160, 160, True, True, False, True),
@@ -29,7 +31,7 @@ CASES = [
     (1, 760, 900, False, False, False, True),      # either height, single
     (1, 1100, 1024, False, True, False, True),
     (1, 1601, 1499, False, False, False, True),
-    (1, 1536, 1600, False, True, True, True),
+    (1, 1536, 1536, False, True, True, True),
 ]
 
 
