@@ -265,20 +265,47 @@ inline size_t galerkin_tile_smem(bool kx, bool ky) {
     return sizeof(double) * (9 * SW * SH + 4 * (SW + 2) * (SH + 2));
 }
 
-/** Single-precision copy of a level's Galerkin stencils (entry k of unknown
- * q at k*N+q) for the centred FP32 cycles: entry 4 holds the row sum of the
- * FP64 stencil, summed in FP64, instead of the diagonal. */
-__global__ void k_cast_stencil(const double *st, float *stf, long N) {
-    for (long q = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; q < N;
-         q += static_cast<long>(gridDim.x) * blockDim.x) {
-        double rs = 0;
+/** One array to round to single precision: a level's Galerkin stencils (entry
+ * k of unknown q at k*N+q) or the weight planes of a transfer, by `blocks`
+ * blocks from `first` on. */
+struct CastJob {
+    const double *src;
+    float *dst;
+    long N;
+    int stencil, first, blocks;
+};
+constexpr int kCastJobs = 32;
+struct CastPlan {
+    int count;
+    CastJob job[kCastJobs];
+};
+
+/** Single-precision copies for the centred FP32 cycles, all levels in one
+ * launch. Entry 4 of a stencil holds the row sum of the FP64 entries, summed in
+ * FP64, instead of the diagonal. Bound by memory: a point's nine loads go out
+ * together (a store between them kept each waiting for the last). The two
+ * systems of a 2048^2 flag: 182 us each in eleven launches for the stencils alone,
+ * 79 us now with the planes; 1024^2, sixteen launches of 3.6 us before. */
+__global__ void __launch_bounds__(256) k_cast_levels(const __grid_constant__ CastPlan p) {
+    int l = 0;
+    while (l + 1 < p.count && static_cast<int>(blockIdx.x) >= p.job[l + 1].first) l++;
+    const double *__restrict__ src = p.job[l].src;
+    float *__restrict__ dst = p.job[l].dst;
+    const long N = p.job[l].N, step = p.job[l].blocks * 256L;
+    const long q0 = (blockIdx.x - p.job[l].first) * 256L + threadIdx.x;
+    if (p.job[l].stencil) {
+        for (long q = q0; q < N; q += step) {
+            double v[9], rs = 0;
 #pragma unroll
-        for (int k = 0; k < 9; k++) {
-            const double v = st[k * N + q];
-            rs += v;
-            if (k != 4) stf[k * N + q] = static_cast<float>(v);
+            for (int k = 0; k < 9; k++) v[k] = src[k * N + q];
+#pragma unroll
+            for (int k = 0; k < 9; k++) rs += v[k];
+#pragma unroll
+            for (int k = 0; k < 9; k++) dst[k * N + q] = static_cast<float>(k == 4 ? rs : v[k]);
         }
-        stf[4 * N + q] = static_cast<float>(rs);
+    } else {
+#pragma unroll 4
+        for (long q = q0; q < N; q += step) dst[q] = static_cast<float>(src[q]);
     }
 }
 
@@ -293,12 +320,6 @@ __global__ void k_smooth(Op op, T *z, const T *b, int m, int n, int pi, int pj) 
     if (i >= m || j >= n) return;
     const int ij = i + m * j;
     z[ij] = gs_update(op, i, j, z, b[ij]);
-}
-
-/** Index i of a periodic direction of size m brought into [0, m). */
-__device__ __forceinline__ int wrap_index(int i, int m) {
-    i %= m;
-    return i < 0 ? i + m : i;
 }
 
 /** Coarse right-hand side b_c = P^T (b - A z), the fine residual formed on
@@ -1147,17 +1168,24 @@ int Multigrid::galerkin_graph() {
 
 int Multigrid::cast_levels() {
     if (!f32_stale) return INCRMT_OK;
-    for (size_t l = 1; l < lev.size(); l++) {
-        MgLevel &C = lev[l];
-        k_cast_stencil<<<cdiv(C.N, 256) < kRedBlocks ? cdiv(C.N, 256) : kRedBlocks, 256, 0, stream>>>(C.st, C.stf, C.N);
+    CastPlan p{};
+    int blocks = 0;
+    const auto flush = [&]() {
+        if (!p.count) return;
+        k_cast_levels<<<blocks, 256, 0, stream>>>(p);
         launches++;
-    }
-    for (size_t l = 0; l + 1 < lev.size(); l++) {
-        const long N = lev[l].planes();
-        k_cast_planes<<<cdiv(N, 256) < kRedBlocks ? cdiv(N, 256) : kRedBlocks, 256, 0, stream>>>(lev[l].Q, lev[l].Qf, N);
-        launches++;
-    }
-    INCRMT_CKL("k_cast_stencil");
+        p.count = blocks = 0;
+    };
+    const auto add = [&](const double *src, float *dst, long N, int stencil) {
+        const int nb = cdiv(N, 256) < 2 * kRedBlocks ? cdiv(N, 256) : 2 * kRedBlocks;
+        p.job[p.count++] = CastJob{src, dst, N, stencil, blocks, nb};
+        blocks += nb;
+        if (p.count == kCastJobs) flush();
+    };
+    for (size_t l = 1; l < lev.size(); l++) add(lev[l].st, lev[l].stf, lev[l].N, 1);
+    for (size_t l = 0; l + 1 < lev.size(); l++) add(lev[l].Q, lev[l].Qf, lev[l].planes(), 0);
+    flush();
+    INCRMT_CKL("k_cast_levels");
     int r = tail_pack<float>();
     if (r) return r;
     f32_stale = false;

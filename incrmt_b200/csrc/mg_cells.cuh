@@ -293,15 +293,15 @@ __global__ void __launch_bounds__(32 * RY, MINB) k_smooth_cells(Op op, const T *
         T *dst = zout + i + static_cast<long>(m) * j;
         *reinterpret_cast<V *>(dst) = V{src[0], src[PL]};
         if (j + 1 < n) *reinterpret_cast<V *>(dst + m) = V{src[2 * PL], src[3 * PL]};
-        return;
-    }
-    for (int r = 2 * HY + (threadIdx.x >> 5); r < 2 * (HY + TY); r += RY) {
-        const int j = 2 * Y + r;
-        if (j >= n) break;
-        const T *src = zs + (r & 1) * 2 * PL + (r >> 1) * RX;
-        for (int t = 2 * HX + (threadIdx.x & 31); t < 2 * (HX + TX); t += 32) {
-            const int i = 2 * X + t;
-            if (i < m) zout[i + static_cast<long>(m) * j] = src[(t & 1) * PL + (t >> 1)];
+    } else {
+        for (int r = 2 * HY + (threadIdx.x >> 5); r < 2 * (HY + TY); r += RY) {
+            const int j = 2 * Y + r;
+            if (j >= n) break;
+            const T *src = zs + (r & 1) * 2 * PL + (r >> 1) * RX;
+            for (int t = 2 * HX + (threadIdx.x & 31); t < 2 * (HX + TX); t += 32) {
+                const int i = 2 * X + t;
+                if (i < m) zout[i + static_cast<long>(m) * j] = src[(t & 1) * PL + (t >> 1)];
+            }
         }
     }
 }

@@ -121,13 +121,6 @@ __global__ void __launch_bounds__(kPX * kPY) k_build_p(Op op, int fm, int fn, in
     for (int r = 0; r < 4; r++) Q[(4 + r) * NC + q] = w[r];
 }
 
-/** Rounds the weight planes to single precision. */
-__global__ void k_cast_planes(const double *Q, float *Qf, long N) {
-    for (long q = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; q < N;
-         q += static_cast<long>(gridDim.x) * blockDim.x)
-        Qf[q] = static_cast<float>(Q[q]);
-}
-
 constexpr int kRX = 32, kRY = 16;  // cells of a block of k_restrict_cells
 
 /** Coarse right-hand side b_c = P^T (b - A z) and cleared coarse iterate, one
