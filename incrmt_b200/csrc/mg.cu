@@ -533,23 +533,6 @@ struct ResPoint<FemOp<double>> {
     }
 };
 
-/** Whether the V-cycles go on after one that left the squared residual rn2, by
- * the tests that follow them on the host: solved, not finite, no longer
- * halving in mixed precision, or at the limit. */
-__device__ __forceinline__ bool loop_goes_on(MgLoop *p, double rn2, double *host) {
-    const double rn = sqrt(rn2), prev = p->prev;
-    const int k = ++p->k;
-    host[0] = rn2;
-    host[1] = k;
-    host[2] = prev;
-    p->prev = rn;
-    return isfinite(rn) && rn > p->tol && !(p->mixed && rn > kMixedContraction * prev) && k < p->maxc;
-}
-
-__global__ void k_loop_begin(MgLoop *p, double tol, double prev, int k, int maxc, int mixed) {
-    *p = MgLoop{tol, prev, k, maxc, mixed};
-}
-
 /** FP64 residual r = b - A z, optionally stored in FP32, and the sum of r^2 in
  * the host's host[0]. Each block takes every gridDim.x-th row, its threads the
  * row's unknowns (coalesced, no index division). Bound by memory once the loads
@@ -557,11 +540,12 @@ __global__ void k_loop_begin(MgLoop *p, double tol, double prev, int k, int maxc
  * -> 101 us (four points 107), FEM 140 -> 108 (two points spill: 187), of 82 and
  * 61 us for the bytes. The total and its way to the host are this launch's too
  * (small grids: 2.1 us, 1.9 for the sum and 3.3 for the copy before, 4.5 now).
- * As the end of a captured loop's body it also decides whether that runs again. */
+ * Solves: MAC 64^2 603 -> 547 us, FEM 193 x 144 1688 -> 1531. A loop inside the
+ * graph, left by this kernel, took as long as a graph launch per cycle (MAC 64^2
+ * on the device 411 us and 410) and 0.05 ms more on a solve's first buffers. */
 template <class Op>
 __global__ void __launch_bounds__(256, 4) k_resnorm(Op op, const double *__restrict__ z, const double *__restrict__ b, int m, int n,
-                                                    float *__restrict__ rf, double *partial, unsigned *ticket, double *host,
-                                                    MgLoop *loop, cudaGraphConditionalHandle body) {
+                                                    float *__restrict__ rf, double *partial, unsigned *ticket, double *host) {
     constexpr int U = Op::kFivePoint ? 2 : 1;
     double acc = 0;
     for (int j = blockIdx.x; j < n; j += gridDim.x)
@@ -579,10 +563,7 @@ __global__ void __launch_bounds__(256, 4) k_resnorm(Op op, const double *__restr
                 }
             }
         }
-    if (grid_sum_256(acc, partial, ticket)) {
-        if (loop) cudaGraphSetConditional(body, loop_goes_on(loop, acc, host));
-        else host[0] = acc;
-    }
+    if (grid_sum_256(acc, partial, ticket)) *host = acc;
 }
 
 /** out = A z. */
@@ -914,9 +895,8 @@ int Multigrid::create(int sys_, int cm_, int cn_, double ax, double bx, double a
     INCRMT_CK(cudaMalloc(&bbuf, sizeof(double) * N));
     INCRMT_CK(cudaMalloc(&zbuf, sizeof(double) * N));
     INCRMT_CK(cudaMalloc(&partial, sizeof(double) * kRedBlocks));
-    INCRMT_CK(cudaMalloc(&dnorm, sizeof(double) * 8 + sizeof(MgLoop)));
+    INCRMT_CK(cudaMalloc(&dnorm, sizeof(double) * 5));
     ticket = reinterpret_cast<unsigned *>(dnorm + 4);
-    loop = reinterpret_cast<MgLoop *>(dnorm + 8);
     INCRMT_CK(cudaMemsetAsync(ticket, 0, sizeof(unsigned), stream));
     INCRMT_CK(cudaMallocHost(&hnorm, sizeof(double) * 4));
     return build_hierarchy();
@@ -1523,12 +1503,10 @@ int Multigrid::norm2_rhs(const double *b, double *out_dev) {
     return INCRMT_OK;
 }
 
-int Multigrid::residual_norm(const double *b, const double *z, float *rf, const cudaGraphConditionalHandle *body) {
+int Multigrid::residual_norm(const double *b, const double *z, float *rf) {
     const int nb = n < kRedBlocks ? n : kRedBlocks;  // blocks over the rows
-    const cudaGraphConditionalHandle h = body ? *body : 0;
-    MgLoop *p = body ? loop : nullptr;
-    if (sys == INCRMT_SYS_MAC) k_resnorm<<<nb, 256, 0, stream>>>(mac64(), z, b, m, n, rf, partial, ticket, hnorm, p, h);
-    else k_resnorm<<<nb, 256, 0, stream>>>(fem64(), z, b, m, n, rf, partial, ticket, hnorm, p, h);
+    if (sys == INCRMT_SYS_MAC) k_resnorm<<<nb, 256, 0, stream>>>(mac64(), z, b, m, n, rf, partial, ticket, hnorm);
+    else k_resnorm<<<nb, 256, 0, stream>>>(fem64(), z, b, m, n, rf, partial, ticket, hnorm);
     launches++;
     INCRMT_CKL("residual norm");
     return INCRMT_OK;
@@ -1543,12 +1521,12 @@ int Multigrid::fetch_norm(double *v) {
 
 /** One V-cycle (FP64, or one FP32 defect-correction step in mixed mode),
  * the FP64 residual norm of the new iterate in hnorm[0]. */
-int Multigrid::vcycle_and_norm(int prec, const double *b, double *d_z, long N, const cudaGraphConditionalHandle *body) {
+int Multigrid::vcycle_and_norm(int prec, const double *b, double *d_z, long N) {
     int r;
     const long long l0 = launches;
     if (prec == INCRMT_PREC_FP64) {
         if ((r = cycle64(0, b, d_z))) return r;
-        if ((r = residual_norm(b, d_z, nullptr, body))) return r;
+        if ((r = residual_norm(b, d_z, nullptr))) return r;
     } else {
         const int nbk = cdiv(N, 256) < kRedBlocks ? cdiv(N, 256) : kRedBlocks;
         k_fill<float><<<nbk, 256, 0, stream>>>(lev[0].zf, N, 0.f);
@@ -1567,7 +1545,7 @@ int Multigrid::vcycle_and_norm(int prec, const double *b, double *d_z, long N, c
             launches += 2;
         }
         INCRMT_CKL("defect correction");
-        if ((r = residual_norm(b, d_z, lev[0].bf, body))) return r;
+        if ((r = residual_norm(b, d_z, lev[0].bf))) return r;
     }
     graph_launches = launches - l0;
     return INCRMT_OK;
@@ -1809,45 +1787,22 @@ int Multigrid::solve_device(const double *d_b, double *d_z, const incrmt_mg_opts
         }
     } else if (prec == INCRMT_PREC_MIXED) {
         if ((r = cast_levels())) return r;
-        if ((r = residual_norm(b, d_z, lev[0].bf, nullptr))) return r;
+        if ((r = residual_norm(b, d_z, lev[0].bf))) return r;
         INCRMT_CK(cudaStreamSynchronize(stream));
         rn2 = hnorm[0];
         rn_prev = std::sqrt(rn2);
     }
-    // V-cycles and their residual norms until one of the tests below ends them,
-    // captured once into a CUDA graph per (precision, b, z): the body of a loop
-    // that the last kernel of each cycle continues or leaves. One launch and one
-    // synchronisation per solve instead of per cycle, a round trip of about
-    // 10 us (MAC 64^2, eight cycles, 603 -> 547 us; FEM 193 x 144, thirteen, 1688
-    // -> 1531), against 0.2 ms more for the first solve with new buffers.
+    // One V-cycle and its residual norm, captured once into a CUDA graph per
+    // (precision, b, z) and replayed per cycle.
     const bool use_graph = !prof;
     auto capture = [&]() -> int {
         if (gexec) { cudaGraphExecDestroy(gexec); gexec = nullptr; }
         cudaGraph_t graph = nullptr;
-        INCRMT_CK(cudaGraphCreate(&graph, 0));
-        cudaGraphConditionalHandle body;
-        cudaGraphNodeParams np = {};
-        cudaGraphNode_t node;
-        cudaError_t ce = cudaGraphConditionalHandleCreate(&body, graph, 1, cudaGraphCondAssignDefault);
-        if (ce == cudaSuccess) {
-            np.type = cudaGraphNodeTypeConditional;
-            np.conditional.handle = body;
-            np.conditional.type = cudaGraphCondTypeWhile;
-            np.conditional.size = 1;
-            ce = cudaGraphAddNode(&node, graph, nullptr, 0, &np);
-        }
-        if (ce == cudaSuccess)
-            ce = cudaStreamBeginCaptureToGraph(stream, np.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                               cudaStreamCaptureModeThreadLocal);
-        if (ce != cudaSuccess) {
-            cudaGraphDestroy(graph);
-            return cuda_status(ce, "capture", __FILE__, __LINE__);
-        }
-        int rc = vcycle_and_norm(cur, b, d_z, N, &body);
-        cudaGraph_t captured = nullptr;
-        ce = cudaStreamEndCapture(stream, &captured);
+        INCRMT_CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+        int rc = vcycle_and_norm(cur, b, d_z, N);
+        cudaError_t ce = cudaStreamEndCapture(stream, &graph);
         if (rc || ce != cudaSuccess) {
-            cudaGraphDestroy(graph);
+            if (ce == cudaSuccess && graph) cudaGraphDestroy(graph);
             if (rc) return rc;
             return cuda_status(ce, "capture", __FILE__, __LINE__);
         }
@@ -1861,18 +1816,13 @@ int Multigrid::solve_device(const double *d_b, double *d_z, const incrmt_mg_opts
         return r;
     while (plain && k < maxc) {
         if (use_graph) {
-            k_loop_begin<<<1, 1, 0, stream>>>(loop, tol, rn_prev, k, maxc, cur == INCRMT_PREC_MIXED);
             INCRMT_CK(cudaGraphLaunch(gexec, stream));
-            INCRMT_CK(cudaStreamSynchronize(stream));
-            rn2 = hnorm[0];
-            launches += 1 + graph_launches * (static_cast<int>(hnorm[1]) - k);
-            k = static_cast<int>(hnorm[1]);
-            rn_prev = hnorm[2];
-        } else {
-            if ((r = vcycle_and_norm(cur, b, d_z, N, nullptr))) return r;
-            INCRMT_CK(cudaStreamSynchronize(stream));
-            rn2 = hnorm[0];
-            k++;
+            launches += graph_launches;
+        } else if ((r = vcycle_and_norm(cur, b, d_z, N))) {
+        INCRMT_CK(cudaStreamSynchronize(stream));
+        rn2 = hnorm[0];
+        k++;
+            return r;
         }
         const double rn = std::sqrt(rn2);
         if (!std::isfinite(rn)) { finite = false; break; }

@@ -25,13 +25,6 @@
 
 namespace incrmt {
 
-/** State of a captured loop of V-cycles: tolerance, last residual norm, cycles
- * so far, their limit, and whether they are defect corrections. */
-struct MgLoop {
-    double tol, prev;
-    int k, maxc, mixed;
-};
-
 struct MgLevel {
     int m = 0, n = 0;
     long N = 0;
@@ -72,7 +65,6 @@ public:
     float *ginvf = nullptr;          // and its FP32 copy
     double *hnorm = nullptr;         // pinned host scalars
     double *dnorm = nullptr;         // device scalars
-    MgLoop *loop = nullptr;          // what ends a captured loop of V-cycles
     unsigned *ticket = nullptr;      // blocks finished in a sum over the grid
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     long long launches = 0;
@@ -100,7 +92,7 @@ public:
     int tail_level = -1;             // first level run by the tail kernel (mg_tail.cuh)
     int tail_max_blocks = 1;         // blocks of its cluster at most
     void *tail_pk = nullptr;         // its levels' packed stencils and weights
-    cudaGraphExec_t gexec = nullptr; // captured loop of V-cycles with their norms
+    cudaGraphExec_t gexec = nullptr; // captured V-cycle + norm
     cudaGraphExec_t setup_exec = nullptr;  // captured rebuild of the coarse levels
     long long setup_launches = 0;
     int gkey_prec = -1;
@@ -188,12 +180,11 @@ private:
     template <class T>
     int tail_launch();
     int tail64();
-    int vcycle_and_norm(int prec, const double *b, double *d_z, long N, const cudaGraphConditionalHandle *body);
+    int vcycle_and_norm(int prec, const double *b, double *d_z, long N);
     int tail32();
     int norm2_rhs(const double *b, double *out_dev);
-    /** ||b - A z||^2 into hnorm[0] (b - A z in FP32 into rf); as the end of a
-     * captured loop's body, also whether that runs again. */
-    int residual_norm(const double *b, const double *z, float *rf, const cudaGraphConditionalHandle *body);
+    /** ||b - A z||^2 into hnorm[0] (b - A z in FP32 into rf). */
+    int residual_norm(const double *b, const double *z, float *rf);
     int fetch_norm(double *v);
     int krylov_alloc();
     /** kr = b - A z (and its FP32 copy into lev[0].bf in mixed precision),
