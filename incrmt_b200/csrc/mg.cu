@@ -323,10 +323,10 @@ __global__ void k_smooth(Op op, T *z, const T *b, int m, int n, int pi, int pj) 
 }
 
 /** Coarse right-hand side b_c = P^T (b - A z), the fine residual formed on
- * the fly; also clears the coarse iterate. */
+ * the fly. */
 template <class Op, class T>
 __global__ void k_restrict(Op op, const T *z, const T *b, int fm, int fn, int px, int py,
-                           bool kx, bool ky, int cm, int cn, T *bc, T *zc, const double *P) {
+                           bool kx, bool ky, int cm, int cn, T *bc, const double *P) {
     const int I = blockIdx.x * blockDim.x + threadIdx.x, J = blockIdx.y * blockDim.y + threadIdx.y;
     if (I >= cm || J >= cn) return;
     const int x0 = kx ? 2 * I - 1 : I, x1 = kx ? 2 * I + 1 : I, y0 = ky ? 2 * J - 1 : J, y1 = ky ? 2 * J + 1 : J;
@@ -341,7 +341,6 @@ __global__ void k_restrict(Op op, const T *z, const T *b, int fm, int fn, int px
             t = add_prod(t, w, residual_at(op, i, j, z, b[f]));
         }
     bc[I + cm * J] = t;
-    zc[I + cm * J] = 0;
 }
 
 /** Coarsest-level solve: `sweeps` four-colour Gauss-Seidel sweeps by one
@@ -780,22 +779,25 @@ cudaError_t set_tail_attr() {
 /** Runs `sweeps` four-colour sweeps on the iterate z. Two sweeps on a grid
  * whose periodic directions have even sizes run as one tile-fused launch that
  * reads z and writes zalt (*res = zalt); otherwise one launch per colour
- * updates z in place (*res = z). When prof is given, each launch is bracketed
+ * updates z in place (*res = z). zero: the sweeps start from 0 and z need not
+ * hold it (tiles then read no iterate). When prof is given, each launch is bracketed
  * by CUDA events and credited with its algorithmic bytes: (units updated) x
  * bytes_per_unit. */
 template <class Op, class T>
 int smooth(Op op, T *z, T *zalt, const T *b, int m, int n, int sweeps, cudaStream_t s, long long &nl, T **res,
-           Multigrid *prof = nullptr, double bytes_per_unit = 0) {
+           bool zero = false, Multigrid *prof = nullptr, double bytes_per_unit = 0) {
     *res = z;
     if (sweeps == 2 && zalt && (!op.px || m % 2 == 0) && (!op.py || n % 2 == 0)) {
-        if (prof) { int r = prof->prof_begin(static_cast<double>(m) * n * 2 * bytes_per_unit); if (r) return r; }
-        smooth_cells(op, z, zalt, b, m, n, s);
+        const double words = zero ? sizeof(T) : 0;  // not read
+        if (prof) { int r = prof->prof_begin(static_cast<double>(m) * n * (2 * bytes_per_unit - words)); if (r) return r; }
+        smooth_cells(op, zero ? static_cast<const T *>(nullptr) : z, zalt, b, m, n, s);
         nl++;
         if (prof) { int r = prof->prof_end(); if (r) return r; }
         INCRMT_CKL("k_smooth_cells");
         *res = zalt;
         return INCRMT_OK;
     }
+    if (zero) INCRMT_CK(cudaMemsetAsync(z, 0, sizeof(T) * m * n, s));
     const int pis[4] = {0, 1, 1, 0}, pjs[4] = {0, 1, 0, 1};
     for (int q = 0; q < sweeps; q++)
         for (int c = 0; c < 4; c++) {
@@ -810,21 +812,21 @@ int smooth(Op op, T *z, T *zalt, const T *b, int m, int n, int sweeps, cudaStrea
     return INCRMT_OK;
 }
 
-/** Coarse right-hand side and cleared coarse iterate: the restriction by
+/** Coarse right-hand side: the restriction by
  * cells, or k_restrict when tiles are off (the identity check of
  * incrmt_mg_set_tiles covers both). */
 template <class Op, class T>
 void restrict_launch(bool tiles, Op op, cudaStream_t s, const T *z, const T *b, int px, int py, const MgLevel &L,
-                     const MgLevel &C, T *bc, T *zc, const T *Q) {
+                     const MgLevel &C, T *bc, const T *Q) {
     const int fm = L.m, fn = L.n, cm = C.m, cn = C.n;
     if (!tiles) {
-        k_restrict<<<grid2(cm, cn), kBlk2, 0, s>>>(op, z, b, fm, fn, px, py, L.kx, L.ky, cm, cn, bc, zc, L.P);
+        k_restrict<<<grid2(cm, cn), kBlk2, 0, s>>>(op, z, b, fm, fn, px, py, L.kx, L.ky, cm, cn, bc, L.P);
         return;
     }
     const dim3 g(cdiv(cm, L.kx ? kRX - 1 : kRX), cdiv(cn, L.ky ? kRY - 1 : kRY)), t(kRX, kRY);
-    if (L.kx && L.ky) k_restrict_cells<Op, T, true, true><<<g, t, 0, s>>>(op, z, b, fm, fn, px, py, cm, cn, bc, zc, Q);
-    else if (L.kx) k_restrict_cells<Op, T, true, false><<<g, t, 0, s>>>(op, z, b, fm, fn, px, py, cm, cn, bc, zc, Q);
-    else k_restrict_cells<Op, T, false, true><<<g, t, 0, s>>>(op, z, b, fm, fn, px, py, cm, cn, bc, zc, Q);
+    if (L.kx && L.ky) k_restrict_cells<Op, T, true, true><<<g, t, 0, s>>>(op, z, b, fm, fn, px, py, cm, cn, bc, Q);
+    else if (L.kx) k_restrict_cells<Op, T, true, false><<<g, t, 0, s>>>(op, z, b, fm, fn, px, py, cm, cn, bc, Q);
+    else k_restrict_cells<Op, T, false, true><<<g, t, 0, s>>>(op, z, b, fm, fn, px, py, cm, cn, bc, Q);
 }
 
 /** z += P z_c. */
@@ -1172,7 +1174,7 @@ int Multigrid::cast_levels() {
     return INCRMT_OK;
 }
 
-int Multigrid::cycle64(int l, const double *b0, double *z0) {
+int Multigrid::cycle64(int l, const double *b0, double *z0, bool zero) {
     if (l > 0 && l == tail_level) return tail64();
     const MgLevel &L = lev[l];
     const double *b = l == 0 ? b0 : L.b;
@@ -1180,6 +1182,7 @@ int Multigrid::cycle64(int l, const double *b0, double *z0) {
     GenOp<double> g; g.m = L.m; g.n = L.n; g.px = px; g.py = py; g.N = L.N; g.st = L.st;
     const bool last = l == static_cast<int>(lev.size()) - 1;
     if (last) {
+        if (zero) INCRMT_CK(cudaMemsetAsync(z, 0, sizeof(double) * L.N, stream));
         if (l == 0) {
             if (sys == INCRMT_SYS_MAC) k_coarse<<<1, 256, 0, stream>>>(mac64(), z, b, L.m, L.n, kCoarseSweeps);
             else k_coarse<<<1, 256, 0, stream>>>(fem64(), z, b, L.m, L.n, kCoarseSweeps);
@@ -1201,25 +1204,25 @@ int Multigrid::cycle64(int l, const double *b0, double *z0) {
     double *cur = z;
     if (l == 0 && sys == INCRMT_SYS_MAC) {
         auto op = mac64();
-        if ((r = smooth(op, z, tiles ? L.z2 : nullptr, b, L.m, L.n, kNu1, stream, launches, &cur, pf, bpu))) return r;
-        restrict_launch(tiles, op, stream, cur, b, px, py, L, C, C.b, C.z, L.Q);
+        if ((r = smooth(op, z, tiles ? L.z2 : nullptr, b, L.m, L.n, kNu1, stream, launches, &cur, zero, pf, bpu))) return r;
+        restrict_launch(tiles, op, stream, cur, b, px, py, L, C, C.b, L.Q);
     } else if (l == 0) {
         auto op = fem64();
-        if ((r = smooth(op, z, tiles ? L.z2 : nullptr, b, L.m, L.n, kNu1, stream, launches, &cur, pf, bpu))) return r;
-        restrict_launch(tiles, op, stream, cur, b, px, py, L, C, C.b, C.z, L.Q);
+        if ((r = smooth(op, z, tiles ? L.z2 : nullptr, b, L.m, L.n, kNu1, stream, launches, &cur, zero, pf, bpu))) return r;
+        restrict_launch(tiles, op, stream, cur, b, px, py, L, C, C.b, L.Q);
     } else {
-        if ((r = smooth(g, z, tiles ? L.z2 : nullptr, b, L.m, L.n, kNu1, stream, launches, &cur))) return r;
-        restrict_launch(tiles, g, stream, cur, b, px, py, L, C, C.b, C.z, L.Q);
+        if ((r = smooth(g, z, tiles ? L.z2 : nullptr, b, L.m, L.n, kNu1, stream, launches, &cur, zero))) return r;
+        restrict_launch(tiles, g, stream, cur, b, px, py, L, C, C.b, L.Q);
     }
     launches++;
     INCRMT_CKL("k_restrict");
-    if ((r = cycle64(l + 1, b0, z0))) return r;
+    if ((r = cycle64(l + 1, b0, z0, true))) return r;
     prolong_launch<double>(stream, cur, px, py, L, C, C.z, L.Q);
     launches++;
     INCRMT_CKL("k_prolong");
     double *alt = !tiles ? nullptr : cur == z ? L.z2 : z, *out = cur;
-    if (l == 0 && sys == INCRMT_SYS_MAC) r = smooth(mac64(), cur, alt, b, L.m, L.n, kNu2, stream, launches, &out, pf, bpu);
-    else if (l == 0) r = smooth(fem64(), cur, alt, b, L.m, L.n, kNu2, stream, launches, &out, pf, bpu);
+    if (l == 0 && sys == INCRMT_SYS_MAC) r = smooth(mac64(), cur, alt, b, L.m, L.n, kNu2, stream, launches, &out, false, pf, bpu);
+    else if (l == 0) r = smooth(fem64(), cur, alt, b, L.m, L.n, kNu2, stream, launches, &out, false, pf, bpu);
     else r = smooth(g, cur, alt, b, L.m, L.n, kNu2, stream, launches, &out);
     if (r) return r;
     if (out != z) INCRMT_CK(cudaMemcpyAsync(z, out, sizeof(double) * L.N, cudaMemcpyDeviceToDevice, stream));
@@ -1272,6 +1275,7 @@ int Multigrid::cycle32(int l) {
     GenOp<float> g; g.m = L.m; g.n = L.n; g.px = px; g.py = py; g.N = L.N; g.st = L.stf;
     const bool last = l == static_cast<int>(lev.size()) - 1;
     if (last) {
+        INCRMT_CK(cudaMemsetAsync(z, 0, sizeof(float) * L.N, stream));
         if (l == 0) {
             if (sys == INCRMT_SYS_MAC) k_coarse<<<1, 256, 0, stream>>>(mac32(), z, b, L.m, L.n, kCoarseSweeps);
             else k_coarse<<<1, 256, 0, stream>>>(fem32(), z, b, L.m, L.n, kCoarseSweeps);
@@ -1287,15 +1291,15 @@ int Multigrid::cycle32(int l) {
     const double bpu = 4.0 * (sys == INCRMT_SYS_MAC ? 5 : 4);  // FP32 words: z, b, coefficients in; z out
     if (l == 0 && sys == INCRMT_SYS_MAC) {
         auto op = mac32();
-        if ((r = smooth(op, z, tiles ? L.zf2 : nullptr, b, L.m, L.n, kNu1, stream, launches, &cur, pf, bpu))) return r;
-        restrict_launch(tiles, op, stream, static_cast<const float *>(cur), b, px, py, L, C, C.bf, C.zf, L.Qf);
+        if ((r = smooth(op, z, tiles ? L.zf2 : nullptr, b, L.m, L.n, kNu1, stream, launches, &cur, true, pf, bpu))) return r;
+        restrict_launch(tiles, op, stream, static_cast<const float *>(cur), b, px, py, L, C, C.bf, L.Qf);
     } else if (l == 0) {
         auto op = fem32();
-        if ((r = smooth(op, z, tiles ? L.zf2 : nullptr, b, L.m, L.n, kNu1, stream, launches, &cur, pf, bpu))) return r;
-        restrict_launch(tiles, op, stream, static_cast<const float *>(cur), b, px, py, L, C, C.bf, C.zf, L.Qf);
+        if ((r = smooth(op, z, tiles ? L.zf2 : nullptr, b, L.m, L.n, kNu1, stream, launches, &cur, true, pf, bpu))) return r;
+        restrict_launch(tiles, op, stream, static_cast<const float *>(cur), b, px, py, L, C, C.bf, L.Qf);
     } else {
-        if ((r = smooth(g, z, tiles ? L.zf2 : nullptr, b, L.m, L.n, kNu1, stream, launches, &cur))) return r;
-        restrict_launch(tiles, g, stream, static_cast<const float *>(cur), b, px, py, L, C, C.bf, C.zf, L.Qf);
+        if ((r = smooth(g, z, tiles ? L.zf2 : nullptr, b, L.m, L.n, kNu1, stream, launches, &cur, true))) return r;
+        restrict_launch(tiles, g, stream, static_cast<const float *>(cur), b, px, py, L, C, C.bf, L.Qf);
     }
     launches++;
     INCRMT_CKL("k_restrict");
@@ -1304,8 +1308,8 @@ int Multigrid::cycle32(int l) {
     launches++;
     INCRMT_CKL("k_prolong");
     float *alt = !tiles ? nullptr : cur == z ? L.zf2 : z, *out = cur;
-    if (l == 0 && sys == INCRMT_SYS_MAC) r = smooth(mac32(), cur, alt, b, L.m, L.n, kNu2, stream, launches, &out, pf, bpu);
-    else if (l == 0) r = smooth(fem32(), cur, alt, b, L.m, L.n, kNu2, stream, launches, &out, pf, bpu);
+    if (l == 0 && sys == INCRMT_SYS_MAC) r = smooth(mac32(), cur, alt, b, L.m, L.n, kNu2, stream, launches, &out, false, pf, bpu);
+    else if (l == 0) r = smooth(fem32(), cur, alt, b, L.m, L.n, kNu2, stream, launches, &out, false, pf, bpu);
     else r = smooth(g, cur, alt, b, L.m, L.n, kNu2, stream, launches, &out);
     if (r) return r;
     if (out != z) INCRMT_CK(cudaMemcpyAsync(z, out, sizeof(float) * L.N, cudaMemcpyDeviceToDevice, stream));
@@ -1529,8 +1533,6 @@ int Multigrid::vcycle_and_norm(int prec, const double *b, double *d_z, long N) {
         if ((r = residual_norm(b, d_z, nullptr))) return r;
     } else {
         const int nbk = cdiv(N, 256) < kRedBlocks ? cdiv(N, 256) : kRedBlocks;
-        k_fill<float><<<nbk, 256, 0, stream>>>(lev[0].zf, N, 0.f);
-        launches++;
         if ((r = cycle32(0))) return r;
         if (zpr) {
             k_add_f32<<<nbk, 256, 0, stream>>>(d_z, lev[0].zf, N);
@@ -1586,15 +1588,11 @@ int Multigrid::krylov_iteration(int prec, double *d_z, long N) {
     const int nbr = n < kRedBlocks ? n : kRedBlocks;
     const int singular = zpr ? 0 : 1;
     if (prec == INCRMT_PREC_FP64) {
-        k_fill<double><<<nbk, 256, 0, stream>>>(ke, N, 0.0);
-        launches++;
-        if ((r = cycle64(0, kr, ke))) return r;
+        if ((r = cycle64(0, kr, ke, true))) return r;
         k_cg_dots<double><<<nbk, 256, 0, stream>>>(ke, kq, N, kpart);
         k_reduce_n<3><<<1, 256, 0, stream>>>(kpart, nbk, ks);
         k_cg_direction<double><<<nbk, 256, 0, stream>>>(ke, kp, N, ks, singular);
     } else {
-        k_fill<float><<<nbk, 256, 0, stream>>>(lev[0].zf, N, 0.f);
-        launches++;
         if ((r = cycle32(0))) return r;
         k_cg_dots<float><<<nbk, 256, 0, stream>>>(lev[0].zf, kq, N, kpart);
         k_reduce_n<3><<<1, 256, 0, stream>>>(kpart, nbk, ks);
@@ -1819,11 +1817,11 @@ int Multigrid::solve_device(const double *d_b, double *d_z, const incrmt_mg_opts
             INCRMT_CK(cudaGraphLaunch(gexec, stream));
             launches += graph_launches;
         } else if ((r = vcycle_and_norm(cur, b, d_z, N))) {
+            return r;
+        }
         INCRMT_CK(cudaStreamSynchronize(stream));
         rn2 = hnorm[0];
         k++;
-            return r;
-        }
         const double rn = std::sqrt(rn2);
         if (!std::isfinite(rn)) { finite = false; break; }
         if (rn <= tol) { conv = true; break; }

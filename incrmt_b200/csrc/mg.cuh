@@ -172,7 +172,9 @@ private:
     /** FP32 copies of the Galerkin stencils, made on the first mixed solve
      * after a rebuild (FP64 solves never read them). */
     int cast_levels();
-    int cycle64(int l, const double *b0, double *z0);
+    /** A V-cycle from level l down on A z = b (level 0: z0, b0); zero: from 0, what z
+     * holds is not read. cycle32 starts from 0 on every level. */
+    int cycle64(int l, const double *b0, double *z0, bool zero = false);
     int cycle32(int l);
     int choose_tail();
     template <class T>

@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(kPX * kPY) k_build_p(Op op, int fm, int fn, in
 
 constexpr int kRX = 32, kRY = 16;  // cells of a block of k_restrict_cells
 
-/** Coarse right-hand side b_c = P^T (b - A z) and cleared coarse iterate, one
+/** Coarse right-hand side b_c = P^T (b - A z), one
  * thread per cell: it forms the residuals of its fine points into shared
  * memory, then sums its coarse point's support with the weights and in the
  * order of k_restrict: the same values. In a halved direction the blocks
@@ -135,7 +135,7 @@ constexpr int kRX = 32, kRY = 16;  // cells of a block of k_restrict_cells
  * 4096^2 solve's four levels FP64 58.8 -> 27.6 on average. */
 template <class Op, class T, bool KX, bool KY>
 __global__ void __launch_bounds__(kRX * kRY) k_restrict_cells(Op op, const T *z, const T *b, int fm, int fn, int px, int py,
-                                                              int cm, int cn, T *bc, T *zc, const T *Q) {
+                                                              int cm, int cn, T *bc, const T *Q) {
     constexpr int NX = KX ? 2 : 1, NY = KY ? 2 : 1;
     __shared__ T rs[NY][NX][kRY][kRX + 1];
     const int cx = cells_of(fm, KX), cy = cells_of(fn, KY);
@@ -189,7 +189,6 @@ __global__ void __launch_bounds__(kRX * kRY) k_restrict_cells(Op op, const T *z,
         add(w2, rs[1][0][ty][tx]);
     }
     bc[I + cm * J] = t;
-    zc[I + cm * J] = 0;
 }
 
 /** Fine correction z += P z_c, one thread per cell; vec: the rows' point pairs
