@@ -42,18 +42,19 @@ __host__ __device__ __forceinline__ int half_floor(int a) { return a >= 0 ? a / 
 __host__ __device__ __forceinline__ int base_of(int i, bool k) { return k ? half_floor(i) : i; }
 
 /** Prolongation weight of fine point (fi,fj) (unwrapped indices) for coarse
- * point (I,J): entry qx+2qy of the point's four stored weights, with (qx,qy)
+ * point (I,J): entry qx+2qy of the point's four weights, with (qx,qy)
  * the coarse point's offset from the point's base; 0 when it is not one of
  * its corners or the point is outside a non-periodic grid. */
-template <class W>
-__device__ __forceinline__ double pweight(const W *P, int fm, int fn, int px, int py, bool kx, bool ky, int fi,
+__device__ __forceinline__ double pweight(const double *Q, int fm, int fn, int px, int py, bool kx, bool ky, int fi,
                                           int fj, int I, int J) {
     const int qx = I - base_of(fi, kx), qy = J - base_of(fj, ky);
     if (qx < 0 || qx > 1 || qy < 0 || qy > 1) return 0;
     bool ok = true;
     const int i = wrap_idx(fi, fm, px, ok), j = wrap_idx(fj, fn, py, ok);
     if (!ok) return 0;
-    return static_cast<double>(P[4 * (static_cast<long>(i) + static_cast<long>(fm) * j) + qx + 2 * qy]);
+    double w[4];
+    plane_weights(Q, cells_of(fm, kx), cells_of(fn, ky), kx, ky, i, j, w);
+    return w[qx + 2 * qy];
 }
 
 }  // namespace
@@ -106,14 +107,14 @@ __global__ void k_fem_coef(const double *rho, int ml, int mf, int nf, double *c,
  * added to the entry of K - (I,J), K running over g's corners. */
 template <class Op>
 __global__ void k_galerkin(Op op, int fm, int fn, int px, int py, bool kx, bool ky, int cm, int cn, double *st,
-                           const double *P) {
+                           const double *Q) {
     const int I = blockIdx.x * blockDim.x + threadIdx.x, J = blockIdx.y * blockDim.y + threadIdx.y;
     if (I >= cm || J >= cn) return;
     double q[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     const int x0 = kx ? 2 * I - 1 : I, x1 = kx ? 2 * I + 1 : I, y0 = ky ? 2 * J - 1 : J, y1 = ky ? 2 * J + 1 : J;
     for (int fj = y0; fj <= y1; fj++)
         for (int fi = x0; fi <= x1; fi++) {
-            const double w = pweight(P, fm, fn, px, py, kx, ky, fi, fj, I, J);
+            const double w = pweight(Q, fm, fn, px, py, kx, ky, fi, fj, I, J);
             if (w == 0) continue;
             bool ok = true;
             const int i = wrap_idx(fi, fm, px, ok), j = wrap_idx(fj, fn, py, ok);
@@ -126,7 +127,8 @@ __global__ void k_galerkin(Op op, int fm, int fn, int px, int py, bool kx, bool 
                     bool okg = true;
                     const int gi = wrap_idx(fi + di, fm, px, okg), gj = wrap_idx(fj + dj, fn, py, okg);
                     if (!okg) continue;
-                    const double *g = P + 4 * (static_cast<long>(gi) + static_cast<long>(fm) * gj);
+                    double g[4];
+                    plane_weights(Q, cells_of(fm, kx), cells_of(fn, ky), kx, ky, gi, gj, g);
                     const int ox = base_of(fi + di, kx) - I, oy = base_of(fj + dj, ky) - J;
                     for (int r = 0; r < 4; r++) {
                         const int kx_ = ox + (r & 1), ky_ = oy + (r >> 1);
@@ -159,7 +161,7 @@ constexpr int kGalRows = 4;  // coarse rows of a tile
  * 2048^2 flag's Galerkin levels 42.1 -> 18.7, FEM 1024^2 152 -> 57. */
 template <class Op, bool KX, bool KY>
 __global__ void __launch_bounds__(32 * kGalRows) k_galerkin_tile(Op op, int fm, int fn, int px, int py, int cm, int cn,
-                                                       double *st, const double *P) {
+                                                       double *st, const double *Q) {
     // The coarsening flags are template parameters: with them every loop
     // below has fixed bounds and every offset of a support point or stencil
     // neighbour relative to the coarse point is a constant, so the nine sums
@@ -185,10 +187,7 @@ __global__ void __launch_bounds__(32 * kGalRows) k_galerkin_tile(Op op, int fm, 
         bool ok = xu <= sxmax + 1 && yu <= symax + 1;
         const int i = wrap_idx(xu, fm, px, ok), j = wrap_idx(yu, fn, py, ok);
         double w[4] = {0, 0, 0, 0};
-        if (ok) {
-            const double *q = P + 4 * (static_cast<long>(i) + static_cast<long>(fm) * j);
-            w[0] = q[0]; w[1] = q[1]; w[2] = q[2]; w[3] = q[3];
-        }
+        if (ok) plane_weights(Q, cells_of(fm, kx), cells_of(fn, ky), kx, ky, i, j, w);
         Ps[4 * t] = w[0]; Ps[4 * t + 1] = w[1]; Ps[4 * t + 2] = w[2]; Ps[4 * t + 3] = w[3];
     }
     for (int t = threadIdx.x; t < SA; t += blockDim.x) {
@@ -326,14 +325,14 @@ __global__ void k_smooth(Op op, T *z, const T *b, int m, int n, int pi, int pj) 
  * the fly. */
 template <class Op, class T>
 __global__ void k_restrict(Op op, const T *z, const T *b, int fm, int fn, int px, int py,
-                           bool kx, bool ky, int cm, int cn, T *bc, const double *P) {
+                           bool kx, bool ky, int cm, int cn, T *bc, const double *Q) {
     const int I = blockIdx.x * blockDim.x + threadIdx.x, J = blockIdx.y * blockDim.y + threadIdx.y;
     if (I >= cm || J >= cn) return;
     const int x0 = kx ? 2 * I - 1 : I, x1 = kx ? 2 * I + 1 : I, y0 = ky ? 2 * J - 1 : J, y1 = ky ? 2 * J + 1 : J;
     T t = 0;
     for (int fj = y0; fj <= y1; fj++)
         for (int fi = x0; fi <= x1; fi++) {
-            const T w = static_cast<T>(pweight(P, fm, fn, px, py, kx, ky, fi, fj, I, J));
+            const T w = static_cast<T>(pweight(Q, fm, fn, px, py, kx, ky, fi, fj, I, J));
             if (w == 0) continue;
             bool ok = true;
             const int i = wrap_idx(fi, fm, px, ok), j = wrap_idx(fj, fn, py, ok);
@@ -820,7 +819,7 @@ void restrict_launch(bool tiles, Op op, cudaStream_t s, const T *z, const T *b, 
                      const MgLevel &C, T *bc, const T *Q) {
     const int fm = L.m, fn = L.n, cm = C.m, cn = C.n;
     if (!tiles) {
-        k_restrict<<<grid2(cm, cn), kBlk2, 0, s>>>(op, z, b, fm, fn, px, py, L.kx, L.ky, cm, cn, bc, L.P);
+        k_restrict<<<grid2(cm, cn), kBlk2, 0, s>>>(op, z, b, fm, fn, px, py, L.kx, L.ky, cm, cn, bc, L.Q);
         return;
     }
     const dim3 g(cdiv(cm, L.kx ? kRX - 1 : kRX), cdiv(cn, L.ky ? kRY - 1 : kRY)), t(kRX, kRY);
@@ -944,9 +943,8 @@ int Multigrid::build_hierarchy() {
     }
     // Prolongation weights of every level but the coarsest (k_build_p).
     for (size_t l = 0; l + 1 < lev.size(); l++) {
-        // the weights and, behind them, their planes in both precisions
-        INCRMT_CK(cudaMalloc(&lev[l].P, sizeof(double) * 4 * lev[l].N + (sizeof(double) + sizeof(float)) * lev[l].planes()));
-        lev[l].Q = lev[l].P + 4 * lev[l].N;
+        // the planes in both precisions
+        INCRMT_CK(cudaMalloc(&lev[l].Q, (sizeof(double) + sizeof(float)) * lev[l].planes()));
         lev[l].Qf = reinterpret_cast<float *>(lev[l].Q + lev[l].planes());
     }
     if (lev.size() > 1 && lev.back().N <= kDirectMax) {
@@ -971,7 +969,7 @@ int Multigrid::build_hierarchy() {
 void Multigrid::destroy() {
     for (auto &L : lev) {
         cudaFree(L.z); cudaFree(L.b); cudaFree(L.st); cudaFree(L.zf); cudaFree(L.bf); cudaFree(L.stf);
-        cudaFree(L.z2); cudaFree(L.zf2); cudaFree(L.P);
+        cudaFree(L.z2); cudaFree(L.zf2); cudaFree(L.Q);
     }
     lev.clear();
     cudaFree(ex); cudaFree(ey); cudaFree(exf); cudaFree(eyf); cudaFree(c); cudaFree(cf);
@@ -1085,17 +1083,17 @@ int Multigrid::galerkin_all() {
             const int cx = cells_of(F.m, F.kx), cy = cells_of(F.n, F.ky);
             const bool both = F.kx && F.ky;
             const dim3 gb(cdiv(cx, both ? kPX - 1 : kPX), cdiv(cy, both ? kPY - 1 : kPY)), tb(kPX, kPY);
-            if (both) k_build_p<OpT, true, true><<<gb, tb, 0, stream>>>(op, F.m, F.n, px, py, C.m, C.n, F.P, F.Q);
-            else if (F.kx) k_build_p<OpT, true, false><<<gb, tb, 0, stream>>>(op, F.m, F.n, px, py, C.m, C.n, F.P, F.Q);
-            else k_build_p<OpT, false, true><<<gb, tb, 0, stream>>>(op, F.m, F.n, px, py, C.m, C.n, F.P, F.Q);
+            if (both) k_build_p<OpT, true, true><<<gb, tb, 0, stream>>>(op, F.m, F.n, px, py, C.m, C.n, F.Q);
+            else if (F.kx) k_build_p<OpT, true, false><<<gb, tb, 0, stream>>>(op, F.m, F.n, px, py, C.m, C.n, F.Q);
+            else k_build_p<OpT, false, true><<<gb, tb, 0, stream>>>(op, F.m, F.n, px, py, C.m, C.n, F.Q);
             if (tiles && F.kx && F.ky)
-                k_galerkin_tile<OpT, true, true><<<gt, 32 * kGalRows, gsm, stream>>>(op, F.m, F.n, px, py, C.m, C.n, C.st, F.P);
+                k_galerkin_tile<OpT, true, true><<<gt, 32 * kGalRows, gsm, stream>>>(op, F.m, F.n, px, py, C.m, C.n, C.st, F.Q);
             else if (tiles && F.kx)
-                k_galerkin_tile<OpT, true, false><<<gt, 32 * kGalRows, gsm, stream>>>(op, F.m, F.n, px, py, C.m, C.n, C.st, F.P);
+                k_galerkin_tile<OpT, true, false><<<gt, 32 * kGalRows, gsm, stream>>>(op, F.m, F.n, px, py, C.m, C.n, C.st, F.Q);
             else if (tiles)
-                k_galerkin_tile<OpT, false, true><<<gt, 32 * kGalRows, gsm, stream>>>(op, F.m, F.n, px, py, C.m, C.n, C.st, F.P);
+                k_galerkin_tile<OpT, false, true><<<gt, 32 * kGalRows, gsm, stream>>>(op, F.m, F.n, px, py, C.m, C.n, C.st, F.Q);
             else
-                k_galerkin<<<gc, kBlk2, 0, stream>>>(op, F.m, F.n, px, py, F.kx, F.ky, C.m, C.n, C.st, F.P);
+                k_galerkin<<<gc, kBlk2, 0, stream>>>(op, F.m, F.n, px, py, F.kx, F.ky, C.m, C.n, C.st, F.Q);
         };
         if (l == 1 && sys == INCRMT_SYS_MAC) {
             build(mac64());
@@ -1457,7 +1455,7 @@ int Multigrid::tail_pack() {
     for (int k = 0; k < p.count; k++) {
         const MgLevel &L = lev[tail_level + k];
         TailPackLevel<T> &t = p.lev[k];
-        t.m = L.m; t.n = L.n; t.kx = L.kx; t.ky = L.ky; t.P = L.P;
+        t.m = L.m; t.n = L.n; t.kx = L.kx; t.ky = L.ky; t.Q = L.Q;
         t.cells = ((L.m + 1) / 2) * ((L.n + 1) / 2);
         if constexpr (sizeof(T) == 8) { t.st = L.st; t.pk = L.pk; }
         else { t.st = L.stf; t.pk = L.pkf; }

@@ -32,9 +32,8 @@ struct MgLevel {
     double *z = nullptr, *b = nullptr, *st = nullptr;  // FP64 arrays (level >= 1)
     float *zf = nullptr, *bf = nullptr, *stf = nullptr;  // FP32 arrays (all levels)
     double *z2 = nullptr;  // second FP64 iterate buffer of the tile smoothers (all levels)
-    double *P = nullptr;   // prolongation to the next level: four weights per unknown (all but the last)
     float *zf2 = nullptr;  // and the FP32 one
-    double *Q = nullptr;   // P's weights as planes over the cells (mg_transfer.cuh), and in FP32
+    double *Q = nullptr;   // weights of the prolongation to the next level, planes over its cells (mg_transfer.cuh), and in FP32
     float *Qf = nullptr;
     /** Elements of the planes. */
     long planes() const {

@@ -271,6 +271,25 @@ __host__ __device__ __forceinline__ long colour_index(int m, int n, int i, int j
     return base + static_cast<long>(j >> 1) * (pi ? m1 : m0) + (i >> 1);
 }
 
+/** Cells of a level along an axis: pairs of points where it is halved. */
+__host__ __device__ __forceinline__ int cells_of(int m, bool k) { return k ? (m + 1) >> 1 : m; }
+
+/** The four prolongation weights of fine point (i,j), w[qx+2qy] for the coarse
+ * point at offset (qx,qy) from the point's base, from the planes Q of a level of
+ * cx x cy cells halved along x (kx) and y (ky); mg_transfer.cuh has the layout.
+ * Without a branch around a load, so that the loads of several points are in
+ * flight together. */
+__device__ __forceinline__ void plane_weights(const double *Q, int cx, int cy, bool kx, bool ky, int i, int j, double w[4]) {
+    const bool pi = kx && (i & 1), pj = ky && (j & 1), odd = pi || pj, all = pi && pj;
+    const long NC = static_cast<long>(cx) * cy;
+    const double *q = Q + (kx ? i >> 1 : i) + static_cast<long>(cx) * (ky ? j >> 1 : j) + (kx && pj ? (pi ? 4 : 2) : 0) * NC;
+    const double v0 = odd ? q[0] : 1.0, v1 = odd ? q[NC] : 0.0;
+    w[0] = v0;
+    w[1] = pi ? v1 : 0.0;
+    w[2] = all ? q[2 * NC] : (pj ? v1 : 0.0);
+    w[3] = all ? q[3 * NC] : 0.0;
+}
+
 /** A Galerkin coarse level: explicit 9-point stencil stored structure-of-
  * arrays, entry k of unknown (i,j) at st[k*N + colour_index(m, n, i, j)]. */
 template <class T>

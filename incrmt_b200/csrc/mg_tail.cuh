@@ -93,7 +93,7 @@ template <class T>
 struct TailPackLevel {
     int m, n, kx, ky, cells;
     const T *st;       // Galerkin stencils (single precision: entry 4 the row sum)
-    const double *P;   // prolongation weights, null on the coarsest level
+    const double *Q;   // prolongation weights (planes), null on the coarsest level
     T *pk;
 };
 template <class T>
@@ -120,10 +120,13 @@ __host__ __device__ constexpr int tail_pj(int c) { return c & 1; }
 __host__ __device__ constexpr int tail_colour(int pi, int pj) { return pj ? (pi ? 1 : 3) : (pi ? 2 : 0); }
 
 /** Prolongation weight e of fine point (i,j), unwrapped; 0 outside. */
-__device__ __forceinline__ double tail_weight(const double *P, int m, int n, int px, int py, int i, int j, int e) {
-    if (i < 0 || i >= m) { if (!px) return 0; i += i < 0 ? m : -m; }
-    if (j < 0 || j >= n) { if (!py) return 0; j += j < 0 ? n : -n; }
-    return P[4 * (i + static_cast<long>(m) * j) + e];
+template <class T>
+__device__ __forceinline__ double tail_weight(const TailPackLevel<T> &L, int px, int py, int i, int j, int e) {
+    if (i < 0 || i >= L.m) { if (!px) return 0; i += i < 0 ? L.m : -L.m; }
+    if (j < 0 || j >= L.n) { if (!py) return 0; j += j < 0 ? L.n : -L.n; }
+    double w[4];
+    plane_weights(L.Q, cells_of(L.m, L.kx), cells_of(L.n, L.ky), L.kx, L.ky, i, j, w);
+    return w[e];
 }
 
 /** Packs the levels' stencils and transfer weights by cell, one thread per
@@ -157,7 +160,7 @@ __global__ void k_tail_pack(const __grid_constant__ TailPack<T> p) {
         pk[(kTailCoef<T> * part + 9) * L.cells] = T(1) / d;
         return;
     }
-    if (!L.P) return;
+    if (!L.Q) return;
     if (part == 4) {
         // Weights of the fine points (x0+u, y0+v) of a coarse point's
         // support: slot 3v+u with both directions halved; with one halved the
@@ -166,13 +169,13 @@ __global__ void k_tail_pack(const __grid_constant__ TailPack<T> p) {
             double w = 0;
             if (L.kx && L.ky) {
                 const int u = e % 3, v = e / 3;
-                w = tail_weight(L.P, L.m, L.n, p.px, p.py, 2 * I - 1 + u, 2 * J - 1 + v, (u == 0) + 2 * (v == 0));
+                w = tail_weight(L, p.px, p.py, 2 * I - 1 + u, 2 * J - 1 + v, (u == 0) + 2 * (v == 0));
             } else if (e < 6) {
                 const int q = e / 3, u = e % 3;
                 if (L.kx && 2 * J + q < L.n)
-                    w = tail_weight(L.P, L.m, L.n, p.px, p.py, 2 * I - 1 + u, 2 * J + q, u == 0);
+                    w = tail_weight(L, p.px, p.py, 2 * I - 1 + u, 2 * J + q, u == 0);
                 if (L.ky && 2 * I + q < L.m)
-                    w = tail_weight(L.P, L.m, L.n, p.px, p.py, 2 * I + q, 2 * J - 1 + u, 2 * (u == 0));
+                    w = tail_weight(L, p.px, p.py, 2 * I + q, 2 * J - 1 + u, 2 * (u == 0));
             }
             pk[(kTailRw<T> + e) * L.cells] = static_cast<T>(w);
         }
@@ -182,7 +185,7 @@ __global__ void k_tail_pack(const __grid_constant__ TailPack<T> p) {
     for (int e = 0; e < 8; e++) {
         const int c = e < 2 ? 2 : (e < 4 ? 3 : 1), r = e < 2 ? e : (e < 4 ? 2 * (e - 2) : e - 4);
         const int i = 2 * I + tail_pi(c), j = 2 * J + tail_pj(c);
-        pk[(kTailPw<T> + e) * L.cells] = i < L.m && j < L.n ? static_cast<T>(L.P[4 * (i + static_cast<long>(L.m) * j) + r]) : T(0);
+        pk[(kTailPw<T> + e) * L.cells] = i < L.m && j < L.n ? static_cast<T>(tail_weight(L, p.px, p.py, i, j, r)) : T(0);
     }
 }
 

@@ -5,27 +5,23 @@
 // A cell is the fine points that share a base coarse point: 2 x 2 where both
 // directions are halved, 2 x 1 or 1 x 2 where one is. Its point on the coarse
 // point has the single weight 1; the others' weights, eight per 2 x 2 cell
-// instead of the sixteen slots of the general array P, are kept as planes over
-// the cells, in each precision:
+// instead of sixteen with four slots per point, are kept as planes over the
+// cells, in each precision:
 //   both halved: 0, 1: corners (0,0), (1,0) of point (1,0); 2, 3: corners
 //     (0,0), (0,1) of point (0,1); 4-7: the four corners of point (1,1);
 //   one halved:  0, 1: corners 0, 1 of the odd point.
-// P (four FP64 weights per point) stays for the Galerkin product.
+// All that needs the weights reads these (plane_weights).
 #pragma once
 #include "mg_ops.cuh"
 
 namespace incrmt {
 namespace {
 
-/** Cells of a level along an axis. */
-__host__ __device__ __forceinline__ int cells_of(int m, bool k) { return k ? (m + 1) >> 1 : m; }
-
 constexpr int kPX = 32, kPY = 8;  // cells of a block of k_build_p
 
 /** Operator-dependent prolongation of a level (black-box multigrid:
- * Dendy, J. Comput. Phys. 48 (1982) 366-386): four weights per fine point,
- * P[4f+qx+2qy] for the coarse point at offset (qx,qy) from the point's base
- * (base_of), and the planes Q. A point on a coarse point takes it with weight
+ * Dendy, J. Comput. Phys. 48 (1982) 366-386), a fine point's weights for the
+ * coarse points about it, as planes Q. A point on a coarse point takes it with weight
  * 1; a point between two coarse points along x takes L/(-C) and R/(-C), L, C, R
  * its stencil summed over the columns left of, through and right of it (the
  * operator collapsed along y), and along y likewise with the rows; a point
@@ -43,8 +39,7 @@ constexpr int kPX = 32, kPY = 8;  // cells of a block of k_build_p
  * thread per point -> here): MAC 4096^2 613 -> 251, its Galerkin levels 37 -> 14
  * each, FEM 1024^2 55 -> 17. */
 template <class Op, bool KX, bool KY>
-__global__ void __launch_bounds__(kPX * kPY) k_build_p(Op op, int fm, int fn, int px, int py, int cm, int cn, double *P,
-                                                       double *Q) {
+__global__ void __launch_bounds__(kPX * kPY) k_build_p(Op op, int fm, int fn, int px, int py, int cm, int cn, double *Q) {
     constexpr bool both = KX && KY;
     __shared__ double wx[2][kPY][kPX + 1], wy[2][kPY][kPX + 1];
     const int cx = cells_of(fm, KX), cy = cells_of(fn, KY);
@@ -78,14 +73,6 @@ __global__ void __launch_bounds__(kPX * kPY) k_build_p(Op op, int fm, int fn, in
     }
     if (Iu >= cx || Ju >= cy) return;
     const long NC = static_cast<long>(cx) * cy, q = I + static_cast<long>(cx) * J;
-    auto put = [&](int ii, int jj, double w0, double w1, double w2, double w3) {
-        double2 *p = reinterpret_cast<double2 *>(P + 4 * (ii + static_cast<long>(fm) * jj));
-        p[0] = make_double2(w0, w1);
-        p[1] = make_double2(w2, w3);
-    };
-    put(i, j, 1, 0, 0, 0);
-    if (KX && i + 1 < fm) put(i + 1, j, x0, x1, 0, 0);
-    if (KY && j + 1 < fn) put(i, j + 1, y0, 0, y1, 0);
     if (!both) {
         Q[q] = KX ? x0 : y0;
         Q[NC + q] = KX ? x1 : y1;
@@ -113,7 +100,6 @@ __global__ void __launch_bounds__(kPX * kPY) k_build_p(Op op, int fm, int fn, in
         if (v1) w[1] = -c1 / a[4];
         if (v2) w[2] = -c2 / a[4];
         if (v1 && v2) w[3] = -c3 / a[4];
-        put(i + 1, j + 1, w[0], w[1], w[2], w[3]);
     }
     Q[q] = x0; Q[NC + q] = x1;
     Q[2 * NC + q] = y0; Q[3 * NC + q] = y1;
