@@ -311,12 +311,61 @@ __global__ void __launch_bounds__(256) k_cast_levels(const __grid_constant__ Cas
 // ---------------------------------------------------------------------------
 // V-cycle kernels.
 
-/** One colour (pi,pj) of a Gauss-Seidel sweep: z = (b - offdiag)/diag. */
+// On a periodic level of odd size the first and last columns (rows) have one
+// colour and are neighbours across the seam. Updated in place by unrelated
+// threads each would see the other's value from before or after at random, so
+// the points of such pairs are updated by one block, which computes all its
+// values before it writes any: every point of a colour sees the values from
+// before the phase, as in the tail. The other points run beside them.
+
+constexpr int kSeamUnits = 128;  // pairs of a block of 256 threads
+
+/** Whether colour (pi,pj) meets itself across the x seam and the y seam. */
+struct Seam {
+    bool x, y;
+    __host__ __device__ Seam(int m, int n, int px, int py, int pi, int pj)
+        : x(px && (m & 1) && pi == 0), y(py && (n & 1) && pj == 0) {}
+    /** Pairs: those of the y seam, then those of the x seam in the rows between. */
+    __host__ __device__ int units(int m, int n, int pi, int pj) const {
+        return (y ? (m - pi + 1) / 2 : 0) + (x ? (n - pj + 1) / 2 - (y ? 2 : 0) : 0);
+    }
+    __device__ bool on(int m, int n, int i, int j) const { return (x && (i == 0 || i == m - 1)) || (y && (j == 0 || j == n - 1)); }
+};
+
+/** The pairs from number t0 on, by a block of 2 kSeamUnits threads. The four
+ * corners of a level odd in both directions are all neighbours: pairs 0 and 1. */
+template <class Op, class T>
+__device__ void seam_update(const Op &op, const Seam &e, T *z, const T *b, int pi, int pj, int t0) {
+    const int m = op.m, n = op.n, q = threadIdx.x + blockDim.x * threadIdx.y;
+    const int t = t0 + q % kSeamUnits, ny = e.y ? (m - pi + 1) / 2 : 0;
+    const bool far = q >= kSeamUnits, in = t < e.units(m, n, pi, pj);
+    int i, j;
+    if (t < ny) {
+        i = !e.x ? 2 * t + pi : (t == 0 ? 0 : (t == 1 ? m - 1 : 2 * (t - 1)));
+        j = far ? n - 1 : 0;
+    } else {
+        i = far ? m - 1 : 0;
+        j = 2 * (t - ny + (e.y ? 1 : 0)) + pj;
+    }
+    T v = 0;
+    if (in) v = gs_update(op, i, j, z, b[i + m * j]);
+    __syncthreads();
+    if (in) z[i + m * j] = v;
+}
+
+/** One colour (pi,pj) of a Gauss-Seidel sweep: z = (b - offdiag)/diag. Rows of
+ * blocks beyond the grid update the pairs across the seams. */
 template <class Op, class T>
 __global__ void k_smooth(Op op, T *z, const T *b, int m, int n, int pi, int pj) {
+    const Seam e(m, n, op.px, op.py, pi, pj);
+    const int rows = (n - pj + 2 * blockDim.y - 1) / (2 * blockDim.y);
+    if (static_cast<int>(blockIdx.y) >= rows) {
+        seam_update(op, e, z, b, pi, pj, kSeamUnits * ((blockIdx.y - rows) * gridDim.x + blockIdx.x));
+        return;
+    }
     const int i = 2 * (blockIdx.x * blockDim.x + threadIdx.x) + pi;
     const int j = 2 * (blockIdx.y * blockDim.y + threadIdx.y) + pj;
-    if (i >= m || j >= n) return;
+    if (i >= m || j >= n || e.on(m, n, i, j)) return;
     const int ij = i + m * j;
     z[ij] = gs_update(op, i, j, z, b[ij]);
 }
@@ -343,17 +392,19 @@ __global__ void k_restrict(Op op, const T *z, const T *b, int fm, int fn, int px
 }
 
 /** Coarsest-level solve: `sweeps` four-colour Gauss-Seidel sweeps by one
- * block, with a block barrier between colours. */
+ * block of 256 threads, with a block barrier between colours. */
 template <class Op, class T>
 __global__ void k_coarse(Op op, T *z, const T *b, int m, int n, int sweeps) {
     const int pis[4] = {0, 1, 1, 0}, pjs[4] = {0, 1, 0, 1};
     for (int s = 0; s < sweeps; s++) {
         for (int c = 0; c < 4; c++) {
             const int mc = (m - pis[c] + 1) / 2, nc = (n - pjs[c] + 1) / 2;
+            const Seam e(m, n, op.px, op.py, pis[c], pjs[c]);
             for (int p = threadIdx.x; p < mc * nc; p += blockDim.x) {
                 const int i = 2 * (p % mc) + pis[c], j = 2 * (p / mc) + pjs[c];
-                z[i + m * j] = gs_update(op, i, j, z, b[i + m * j]);
+                if (!e.on(m, n, i, j)) z[i + m * j] = gs_update(op, i, j, z, b[i + m * j]);
             }
+            for (int t = 0; t < e.units(m, n, pis[c], pjs[c]); t += kSeamUnits) seam_update(op, e, z, b, pis[c], pjs[c], t);
             __syncthreads();
         }
     }
@@ -803,7 +854,9 @@ int smooth(Op op, T *z, T *zalt, const T *b, int m, int n, int sweeps, cudaStrea
             const int mc = (m - pis[c] + 1) / 2, nc = (n - pjs[c] + 1) / 2;
             if (mc <= 0 || nc <= 0) continue;
             if (prof) { int r = prof->prof_begin(static_cast<double>(mc) * nc * bytes_per_unit); if (r) return r; }
-            k_smooth<Op, T><<<grid2(mc, nc), kBlk2, 0, s>>>(op, z, b, m, n, pis[c], pjs[c]);
+            dim3 grid = grid2(mc, nc);
+            grid.y += cdiv(cdiv(Seam(m, n, op.px, op.py, pis[c], pjs[c]).units(m, n, pis[c], pjs[c]), kSeamUnits), grid.x);
+            k_smooth<Op, T><<<grid, kBlk2, 0, s>>>(op, z, b, m, n, pis[c], pjs[c]);
             nl++;
             if (prof) { int r = prof->prof_end(); if (r) return r; }
         }
