@@ -488,6 +488,51 @@ __global__ void k_ls_store_status(LsGrid g, const LsObj *ob, const LsWin *win) {
     ob[blockIdx.z].s[ij] = ob[blockIdx.z].ia[ij];
 }
 
+/** The sums of the extrapolation's fit over the points of a window, at offset
+ * (di,dj) with weight w and values (vx,vy), and what follows from them. Every
+ * rounding is written out: the sweeps stop when no value changes, so all loops
+ * that evaluate a point have to give it the same bits. */
+struct ExtFit {
+    double sw, sx, sy, sxx, sxy, syy;
+    __device__ __forceinline__ void clear() { sw = sx = sy = sxx = sxy = syy = 0; }
+    __device__ __forceinline__ void moments(int di, int dj, double w) {
+        const double wi = __dmul_rn(w, di), wj = __dmul_rn(w, dj);
+        sw = __dadd_rn(sw, w);
+        sx = __dadd_rn(sx, wi);
+        sy = __dadd_rn(sy, wj);
+        sxx = __fma_rn(di * di, w, sxx);
+        sxy = dj == 1 ? __dadd_rn(sxy, wi) : (di == 1 ? __dadd_rn(sxy, wj) : __fma_rn(di * dj, w, sxy));
+        syy = __fma_rn(dj * dj, w, syy);
+    }
+    static __device__ __forceinline__ void values(int di, int dj, double w, double vx, double vy, double acc[6]) {
+        const double wi = __dmul_rn(w, di), wj = __dmul_rn(w, dj);
+        acc[0] = __fma_rn(w, vx, acc[0]);
+        acc[1] = __fma_rn(wi, vx, acc[1]);
+        acc[2] = __fma_rn(wj, vx, acc[2]);
+        acc[3] = __fma_rn(w, vy, acc[3]);
+        acc[4] = __fma_rn(wi, vy, acc[4]);
+        acc[5] = __fma_rn(wj, vy, acc[5]);
+    }
+    static __device__ __forceinline__ double minor(double a, double b, double c, double d) {
+        return __fma_rn(a, b, -__dmul_rn(c, d));
+    }
+    __device__ __forceinline__ double det() const {
+        double t = __fma_rn(__dmul_rn(sx, sx), syy, __dmul_rn(sw, minor(sxy, sxy, sxx, syy)));
+        t = __fma_rn(-__dmul_rn(2 * sx, sxy), sy, t);
+        return __fma_rn(__dmul_rn(sy, sy), sxx, t);
+    }
+    /** The coefficients al, be, ga of the fit's value at the point. */
+    __device__ __forceinline__ void solve(double det, double c[3]) const {
+        const double id = 1 / det;
+        c[0] = __dmul_rn(minor(sxy, sxy, sxx, syy), id);
+        c[1] = __dmul_rn(minor(sx, syy, sxy, sy), id);
+        c[2] = __dmul_rn(minor(sxx, sy, sxy, sx), id);
+    }
+    static __device__ __forceinline__ double value(const double *acc, const double c[3]) {
+        return __fma_rn(acc[2], c[2], __fma_rn(acc[0], c[0], __dmul_rn(acc[1], c[1])));
+    }
+};
+
 /** Weighted least-squares extrapolation of (nX,nY) at one band point outside
  * the solid (traverse::extrapolate, traverse.hh:169-231): linear fit over the
  * band neighbours with smaller phi inside a (2r+1)^2 window, weighted by the
@@ -498,11 +543,12 @@ __device__ bool ls_extrap_point(const LsGrid &g, const int *s, const double *phi
                                 const double *cx, const double *cy, int i, int j, double &ox, double &oy) {
     const int P = g.P, ij = j * P + i;
     const double pp = phi[ij];
-    double sw, sx, sy, sxx, sxy, syy, det, acc[6];
+    ExtFit f;
+    double det, acc[6], c[3];
     if (i >= 3 && j >= 3 && i + 3 < g.mL && j + 3 < g.nL) {
         // The radius-3 window lies inside the grid: unrolled, so the status
         // and phi loads of all 49 points issue together. Same sums, same order.
-        sw = sx = sy = sxx = sxy = syy = 0;
+        f.clear();
 #pragma unroll
         for (int k = 0; k < 6; k++) acc[k] = 0;
 #pragma unroll
@@ -520,24 +566,16 @@ __device__ bool ls_extrap_point(const LsGrid &g, const int *s, const double *phi
                 const int q = ij + dj * P + di, st = sq[di + 3];
                 if (st < 2 || st > 5 || !(w[di + 3] < pp)) continue;
                 const double ww = pp - w[di + 3];
-                sw += ww;
-                sx += di * ww;
-                sy += dj * ww;
-                sxx += di * di * ww;
-                sxy += di * dj * ww;
-                syy += dj * dj * ww;
+                f.moments(di, dj, ww);
                 const double vx = st <= 3 ? nX[q] : cx[q], vy = st <= 3 ? nY[q] : cy[q];
-                acc[0] += ww * vx; acc[1] += ww * di * vx; acc[2] += ww * dj * vx;
-                acc[3] += ww * vy; acc[4] += ww * di * vy; acc[5] += ww * dj * vy;
+                ExtFit::values(di, dj, ww, vx, vy, acc);
             }
         }
-        det = sw * (sxy * sxy - sxx * syy) + sx * sx * syy - 2 * sx * sxy * sy + sy * sy * sxx;
+        det = f.det();
         if (!(fabs(det) < 1e-10)) {
-            det = 1 / det;
-            const double al = (sxy * sxy - sxx * syy) * det, be = (sx * syy - sxy * sy) * det,
-                         ga = (sxx * sy - sxy * sx) * det;
-            ox = acc[0] * al + acc[1] * be + acc[2] * ga;
-            oy = acc[3] * al + acc[4] * be + acc[5] * ga;
+            f.solve(det, c);
+            ox = ExtFit::value(acc, c);
+            oy = ExtFit::value(acc + 3, c);
             return true;
         }
     }
@@ -545,7 +583,7 @@ __device__ bool ls_extrap_point(const LsGrid &g, const int *s, const double *phi
     do {
         const int ilo = i <= r ? -i : -r, ihi = i + r >= g.mL ? g.mL - 1 - i : r;
         const int jlo = j <= r ? -j : -r, jhi = j + r >= g.nL ? g.nL - 1 - j : r;
-        sw = sx = sy = sxx = sxy = syy = 0;
+        f.clear();
         for (int k = 0; k < 6; k++) acc[k] = 0;
         for (int dj = jlo; dj <= jhi; dj++)
             for (int di = ilo; di <= ihi; di++) {
@@ -554,24 +592,17 @@ __device__ bool ls_extrap_point(const LsGrid &g, const int *s, const double *phi
                 double w = phi[q];
                 if (!(w < pp)) continue;
                 w = pp - w;
-                sw += w;
-                sx += di * w;
-                sy += dj * w;
-                sxx += di * di * w;
-                sxy += di * dj * w;
-                syy += dj * dj * w;
+                f.moments(di, dj, w);
                 const double vx = sq <= 3 ? nX[q] : cx[q], vy = sq <= 3 ? nY[q] : cy[q];
-                acc[0] += w * vx; acc[1] += w * di * vx; acc[2] += w * dj * vx;
-                acc[3] += w * vy; acc[4] += w * di * vy; acc[5] += w * dj * vy;
+                ExtFit::values(di, dj, w, vx, vy, acc);
             }
-        det = sw * (sxy * sxy - sxx * syy) + sx * sx * syy - 2 * sx * sxy * sy + sy * sy * sxx;
+        det = f.det();
         r++;
     } while (fabs(det) < 1e-10 && r <= 7);
     if (fabs(det) < 1e-10) return false;
-    det = 1 / det;
-    const double al = (sxy * sxy - sxx * syy) * det, be = (sx * syy - sxy * sy) * det, ga = (sxx * sy - sxy * sx) * det;
-    ox = acc[0] * al + acc[1] * be + acc[2] * ga;
-    oy = acc[3] * al + acc[4] * be + acc[5] * ga;
+    f.solve(det, c);
+    ox = ExtFit::value(acc, c);
+    oy = ExtFit::value(acc + 3, c);
     return true;
 }
 
@@ -950,11 +981,10 @@ __global__ void __launch_bounds__(kFimThreads, 1) k_ls_extrap_tiles(LsGrid g, co
                     const int q = work[t], lx = q % REG, ly = q / REG;
                     if (lx < ring || lx >= REG - ring || ly < ring || ly >= REG - ring) continue;
                     const double pp = ph[q];
-                    double acc[6] = {0, 0, 0, 0, 0, 0}, al, be, ga;
+                    double acc[6] = {0, 0, 0, 0, 0, 0}, c[3];
                     if (k == 0) {
-                        // with the fit's moments (the loop of ls_extrap_point,
-                        // so that every sum rounds as there)
-                        double sw = 0, sx = 0, sy = 0, sxx = 0, sxy = 0, syy = 0;
+                        ExtFit f;
+                        f.clear();
 #pragma unroll
                         for (int dj = -3; dj <= 3; dj++)
 #pragma unroll
@@ -963,23 +993,15 @@ __global__ void __launch_bounds__(kFimThreads, 1) k_ls_extrap_tiles(LsGrid g, co
                                 const double p = ph[e];
                                 if (!(p < pp)) continue;
                                 const double ww = pp - p;
-                                sw += ww;
-                                sx += di * ww;
-                                sy += dj * ww;
-                                sxx += di * di * ww;
-                                sxy += di * dj * ww;
-                                syy += dj * dj * ww;
-                                const double vx = cx[e], vy = cy[e];
-                                acc[0] += ww * vx; acc[1] += ww * di * vx; acc[2] += ww * dj * vx;
-                                acc[3] += ww * vy; acc[4] += ww * di * vy; acc[5] += ww * dj * vy;
+                                f.moments(di, dj, ww);
+                                ExtFit::values(di, dj, ww, cx[e], cy[e], acc);
                             }
-                        double det = sw * (sxy * sxy - sxx * syy) + sx * sx * syy - 2 * sx * sxy * sy + sy * sy * sxx;
+                        const double det = f.det();
                         if (fabs(det) < 1e-10) flags[11] = 1;
-                        det = 1 / det;
-                        al = (sxy * sxy - sxx * syy) * det; be = (sx * syy - sxy * sy) * det; ga = (sxx * sy - sxy * sx) * det;
-                        fit[t] = al;
-                        fit[NL + t] = be;
-                        fit[2 * NL + t] = ga;
+                        f.solve(det, c);
+                        fit[t] = c[0];
+                        fit[NL + t] = c[1];
+                        fit[2 * NL + t] = c[2];
                     } else {
 #pragma unroll 1
                         for (int dj = -3; dj <= 3; dj++)
@@ -988,13 +1010,11 @@ __global__ void __launch_bounds__(kFimThreads, 1) k_ls_extrap_tiles(LsGrid g, co
                                 const int e = q + dj * REG + di;
                                 const double p = ph[e];
                                 if (!(p < pp)) continue;
-                                const double ww = pp - p, vx = cx[e], vy = cy[e];
-                                acc[0] += ww * vx; acc[1] += ww * di * vx; acc[2] += ww * dj * vx;
-                                acc[3] += ww * vy; acc[4] += ww * di * vy; acc[5] += ww * dj * vy;
+                                ExtFit::values(di, dj, pp - p, cx[e], cy[e], acc);
                             }
-                        al = fit[t]; be = fit[NL + t]; ga = fit[2 * NL + t];
+                        c[0] = fit[t]; c[1] = fit[NL + t]; c[2] = fit[2 * NL + t];
                     }
-                    const double ox = acc[0] * al + acc[1] * be + acc[2] * ga, oy = acc[3] * al + acc[4] * be + acc[5] * ga;
+                    const double ox = ExtFit::value(acc, c), oy = ExtFit::value(acc + 3, c);
                     if ((ox != cx[q] || oy != cy[q]) && lx >= E::kHalo && lx < E::kHalo + TILE && ly >= E::kHalo &&
                         ly < E::kHalo + TILE)
                         ch = true;
