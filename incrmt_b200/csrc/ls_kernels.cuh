@@ -39,7 +39,7 @@ struct LsGrid {
 
 /** Level-set arrays of one object. The batched kernels below take an array
  * of these and treat blockIdx.z as the object index; the cooperative ones
- * take a combined point list whose entries carry their object index, so
+ * take a combined list of tiles whose entries carry their object index, so
  * every object's band is rebuilt (or extrapolated) in the same launches. */
 struct LsObj {
     double *phi;             // level set (ghosted grid, pitch P)
@@ -488,10 +488,15 @@ __global__ void k_ls_store_status(LsGrid g, const LsObj *ob, const LsWin *win) {
     ob[blockIdx.z].s[ij] = ob[blockIdx.z].ia[ij];
 }
 
-/** The sums of the extrapolation's fit over the points of a window, at offset
- * (di,dj) with weight w and values (vx,vy), and what follows from them. Every
+/** Weighted least-squares extrapolation of the reference map at a band point
+ * outside the solid (traverse::extrapolate, traverse.hh:169-231): a linear fit
+ * over the band neighbours with smaller phi in a (2r+1)^2 window, weighted by the
+ * phi difference w; the window grows from r = 3 to kExtMaxRadius while the system
+ * is singular. Here the sums over the points at offsets (di,dj) with values
+ * (vx,vy), and what follows from them. Every
  * rounding is written out: the sweeps stop when no value changes, so all loops
  * that evaluate a point have to give it the same bits. */
+constexpr int kExtMaxRadius = 7;
 struct ExtFit {
     double sw, sx, sy, sxx, sxy, syy;
     __device__ __forceinline__ void clear() { sw = sx = sy = sxx = sxy = syy = 0; }
@@ -521,6 +526,7 @@ struct ExtFit {
         t = __fma_rn(-__dmul_rn(2 * sx, sxy), sy, t);
         return __fma_rn(__dmul_rn(sy, sy), sxx, t);
     }
+    static __device__ __forceinline__ bool singular(double det) { return fabs(det) < 1e-10; }
     /** The coefficients al, be, ga of the fit's value at the point. */
     __device__ __forceinline__ void solve(double det, double c[3]) const {
         const double id = 1 / det;
@@ -533,119 +539,14 @@ struct ExtFit {
     }
 };
 
-/** Weighted least-squares extrapolation of (nX,nY) at one band point outside
- * the solid (traverse::extrapolate, traverse.hh:169-231): linear fit over the
- * band neighbours with smaller phi inside a (2r+1)^2 window, weighted by the
- * phi difference; the window grows from r=3 to r=7 while the system is
- * singular. Values of points inside the solid come from nX/nY, of points
- * outside from the current iterate (cx,cy). Returns false when singular. */
-__device__ bool ls_extrap_point(const LsGrid &g, const int *s, const double *phi, const double *nX, const double *nY,
-                                const double *cx, const double *cy, int i, int j, double &ox, double &oy) {
-    const int P = g.P, ij = j * P + i;
-    const double pp = phi[ij];
-    ExtFit f;
-    double det, acc[6], c[3];
-    if (i >= 3 && j >= 3 && i + 3 < g.mL && j + 3 < g.nL) {
-        // The radius-3 window lies inside the grid: unrolled, so the status
-        // and phi loads of all 49 points issue together. Same sums, same order.
-        f.clear();
-#pragma unroll
-        for (int k = 0; k < 6; k++) acc[k] = 0;
-#pragma unroll
-        for (int dj = -3; dj <= 3; dj++) {
-            int sq[7];
-            double w[7];
-#pragma unroll
-            for (int di = -3; di <= 3; di++) {
-                const int q = ij + dj * P + di;
-                sq[di + 3] = s[q];
-                w[di + 3] = phi[q];
-            }
-#pragma unroll
-            for (int di = -3; di <= 3; di++) {
-                const int q = ij + dj * P + di, st = sq[di + 3];
-                if (st < 2 || st > 5 || !(w[di + 3] < pp)) continue;
-                const double ww = pp - w[di + 3];
-                f.moments(di, dj, ww);
-                const double vx = st <= 3 ? nX[q] : cx[q], vy = st <= 3 ? nY[q] : cy[q];
-                ExtFit::values(di, dj, ww, vx, vy, acc);
-            }
-        }
-        det = f.det();
-        if (!(fabs(det) < 1e-10)) {
-            f.solve(det, c);
-            ox = ExtFit::value(acc, c);
-            oy = ExtFit::value(acc + 3, c);
-            return true;
-        }
-    }
-    int r = 3;
-    do {
-        const int ilo = i <= r ? -i : -r, ihi = i + r >= g.mL ? g.mL - 1 - i : r;
-        const int jlo = j <= r ? -j : -r, jhi = j + r >= g.nL ? g.nL - 1 - j : r;
-        f.clear();
-        for (int k = 0; k < 6; k++) acc[k] = 0;
-        for (int dj = jlo; dj <= jhi; dj++)
-            for (int di = ilo; di <= ihi; di++) {
-                const int q = ij + dj * P + di, sq = s[q];
-                if (sq < 2 || sq > 5) continue;
-                double w = phi[q];
-                if (!(w < pp)) continue;
-                w = pp - w;
-                f.moments(di, dj, w);
-                const double vx = sq <= 3 ? nX[q] : cx[q], vy = sq <= 3 ? nY[q] : cy[q];
-                ExtFit::values(di, dj, w, vx, vy, acc);
-            }
-        det = f.det();
-        r++;
-    } while (fabs(det) < 1e-10 && r <= 7);
-    if (fabs(det) < 1e-10) return false;
-    f.solve(det, c);
-    ox = ExtFit::value(acc, c);
-    oy = ExtFit::value(acc + 3, c);
-    return true;
-}
-
-/** Appends (ij, object) to the combined point list if it has room;
- * flags an overflow otherwise (the list is sized for every point of every
- * object, so this only guards the bound). */
-__device__ __forceinline__ void ls_list_push(int *list, int *list_k, int *count, int cap, int *overflow, int ij,
+/** Appends (tile, object) to the combined list if it has room; flags an
+ * overflow otherwise (the list is sized for every point of every object, so
+ * this only guards the bound). */
+__device__ __forceinline__ void ls_list_push(int *list, int *list_k, int *count, int cap, int *overflow, int tile,
                                              int k) {
     const int t = atomicAdd(count, 1);
-    if (t < cap) { list[t] = ij; list_k[t] = k; }
+    if (t < cap) { list[t] = tile; list_k[t] = k; }
     else atomicExch(overflow, 1);
-}
-
-/** Lists the band points outside each solid (status 4 or 5). */
-__global__ void k_ls_collect_outside(LsGrid g, const LsObj *ob, const LsWin *win, int *list, int *list_k, int *count, int cap,
-                                     int *overflow) {
-    int i, j;
-    if (!ls_point(g, win, i, j)) return;
-    const int ij = j * g.P + i, st = ob[blockIdx.z].s[ij];
-    if (st == 4 || st == 5) ls_list_push(list, list_k, count, cap, overflow, ij, blockIdx.z);
-}
-
-/** Starts the extrapolation: both buffers of every listed point hold its
- * current reference map. Only listed points are ever read as iterates. */
-__global__ void k_ls_extrap_init(const LsObj *ob, const int *list, const int *list_k, const int *countp, int cap) {
-    const int count = min(*countp, cap);
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < count; t += gridDim.x * blockDim.x) {
-        const LsObj &o = ob[list_k[t]];
-        const int ij = list[t];
-        o.a[ij] = o.b[ij] = o.nX[ij];
-        o.c[ij] = o.d[ij] = o.nY[ij];
-    }
-}
-
-/** Stores the extrapolated values of the listed points into nX, nY. */
-__global__ void k_ls_extrap_store(const LsObj *ob, const int *list, const int *list_k, const int *countp, int cap) {
-    const int count = min(*countp, cap);
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < count; t += gridDim.x * blockDim.x) {
-        const LsObj &o = ob[list_k[t]];
-        const int ij = list[t];
-        o.nX[ij] = o.a[ij];
-        o.nY[ij] = o.c[ij];
-    }
 }
 
 }  // namespace incrmt
@@ -714,7 +615,6 @@ __global__ void k_ls_collect_tiles(LsGrid g, const LsObj *ob, const LsWin *win, 
 /** Threads per block of the cooperative sweeps: one block per SM (the grid
  * barrier costs more with more blocks). */
 constexpr int kFimThreads = 1024;
-constexpr int kExtrapThreads = 512;
 
 /** The march's staging: tiles of TILE x TILE points, SWEEPS sweeps between grid
  * barriers, the halo they need (the stencil and its change marks reach two
@@ -901,45 +801,67 @@ __global__ void __launch_bounds__(kFimThreads, 1) k_ls_fim_coop(LsGrid g, const 
 /** The extrapolation's staging, as Fim: the fit reaches three points. */
 template <int TILE, int SWEEPS>
 struct Ext {
+    static_assert(SWEEPS & 1, "the last sweep writes the second buffer, as a single one does");
+    static_assert(3 * SWEEPS >= kExtMaxRadius, "the halo holds the widest window");
     static constexpr int kHalo = 3 * SWEEPS, kReg = TILE + 2 * kHalo, kPoints = kReg * kReg, kRound = (kPoints + 31) & ~31;
     // listed points: those a sweep may evaluate (three from the region's edge)
     static constexpr int kList = (kReg - 6) * (kReg - 6);
     static constexpr size_t kSmem = kPoints * 5 * sizeof(double) + kList * (3 * sizeof(double) + sizeof(short));
 };
 
-/** All sweeps of the extrapolation wavefront in one cooperative launch, staged
- * like the march (k_ls_fim_coop): the fit's moments depend on the level set
- * alone and are formed by the first sweep of a batch; the others only sum the
- * values of the 7 x 7 window. A point whose window of radius 3 gives a singular
- * fit raises flags[11]: the caller starts over with k_ls_extrap_coop, which
- * widens the window. The first batch reads the reference map itself.
- * flags[0..2], [3] and [4] as in k_ls_fim_coop.
- *
- * Bound by the window sums of the busiest SM. Measured (B200, us per call, one
- * sweep per barrier over global memory -> here): rotor 128^2 266 -> 108, 1024^2
- * 288 -> 107; 32 bodies 1024 x 2048 377 -> 271; flag 2048^2 469 -> 211. */
-template <int TILE, int SWEEPS>
-__global__ void __launch_bounds__(kFimThreads, 1) k_ls_extrap_tiles(LsGrid g, const LsObj *ob, const LsWin *win, const int *list,
-                                                                    const int *list_k, const int *countp, int cap, int *flags,
-                                                                    int max_sweeps) {
+/** The fit at point q of a staged tile of row length reg, whose window grows
+ * while it is singular (points outside the grid or the band hold kUnset); false
+ * where it stays so. */
+__device__ __forceinline__ bool ext_widen(const double *ph, const double *cx, const double *cy, int q, int reg, double &ox,
+                                          double &oy) {
+    const double pp = ph[q];
+    for (int r = 3; r <= kExtMaxRadius; r++) {
+        ExtFit f;
+        f.clear();
+        double acc[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll 1
+        for (int dj = -r; dj <= r; dj++)
+#pragma unroll 1
+            for (int di = -r; di <= r; di++) {
+                const int e = q + dj * reg + di;
+                const double p = ph[e];
+                if (!(p < pp)) continue;
+                f.moments(di, dj, pp - p);
+                ExtFit::values(di, dj, pp - p, cx[e], cy[e], acc);
+            }
+        const double det = f.det();
+        if (ExtFit::singular(det)) continue;
+        double c[3];
+        f.solve(det, c);
+        ox = ExtFit::value(acc, c);
+        oy = ExtFit::value(acc + 3, c);
+        return true;
+    }
+    return false;
+}
+
+/** The batches of k_ls_extrap_tiles: the sweeps made until nothing changed, or
+ * minus one if they run out or a fit is singular. */
+template <int TILE, int SWEEPS, bool WIDE>
+__device__ __forceinline__ int ext_batches(const LsGrid &g, const LsObj *ob, const LsWin *win, const int *list, const int *list_k,
+                                           int count, int *flags, int max_sweeps) {
     namespace cg = cooperative_groups;
     cg::grid_group grid = cg::this_grid();
     using E = Ext<TILE, SWEEPS>;
-    constexpr int REG = E::kReg, RR = E::kPoints, NL = E::kList;
+    constexpr int REG = E::kReg, RR = E::kPoints, NL = E::kList, kRun = WIDE ? 1 : SWEEPS;
     extern __shared__ __align__(16) double ext_smem[];
     double *ph = ext_smem, *xa = ph + RR, *ya = xa + RR, *xb = ya + RR, *yb = xb + RR, *fit = yb + RR;
     unsigned short *work = reinterpret_cast<unsigned short *>(fit + 3 * NL);
     __shared__ int nwork;
-    const int tid = threadIdx.x, count = min(*countp, cap);
-    bool done = false;
-    int it0 = 0;
-    for (int batch = 0; it0 < max_sweeps; batch++, it0 += SWEEPS) {
+    const int tid = threadIdx.x;
+    constexpr int kFirst = WIDE ? 1 : 0;
+    for (int it0 = 0, batch = kFirst; it0 < max_sweeps; batch++, it0 += kRun) {
         if (blockIdx.x == 0 && tid == 0) flags[(batch + 1) % 3] = 0;
         const bool odd = batch & 1;
         for (int tile = blockIdx.x; tile < count; tile += gridDim.x) {
             const LsObj &o = ob[list_k[tile]];
             const LsWin w = win[list_k[tile]];
-            const double *gx = batch == 0 ? o.nX : (odd ? o.b : o.a), *gy = batch == 0 ? o.nY : (odd ? o.d : o.c);
+            const double *gx = batch == kFirst ? o.nX : (odd ? o.b : o.a), *gy = batch == kFirst ? o.nY : (odd ? o.d : o.c);
             const int x0 = w.x0 + (list[tile] & 0xffff) * TILE - E::kHalo;
             const int y0 = w.y0 + (list[tile] >> 16) * TILE - E::kHalo;
             const int xe = min(w.x1, g.mL), ye = min(w.y1, g.nL);
@@ -966,55 +888,66 @@ __global__ void __launch_bounds__(kFimThreads, 1) k_ls_extrap_tiles(LsGrid g, co
                     ya[t] = yb[t] = y;
                 }
                 // (outside the window the band has no points of this object)
-                fim_push(out && lx >= 3 && lx < REG - 3 && ly >= 3 && ly < REG - 3, t, work, &nwork);
+                constexpr int kEdge = WIDE ? E::kHalo : 3;
+                fim_push(out && lx >= kEdge && lx < REG - kEdge && ly >= kEdge && ly < REG - kEdge, t, work, &nwork);
             }
             __syncthreads();
             const int nw = nwork;
             int mask = 0;
 #pragma unroll 1
-            for (int k = 0; k < SWEEPS; k++) {
+            for (int k = 0; k < kRun; k++) {
                 const int ring = 3 * (k + 1);
                 const double *cx = k & 1 ? xb : xa, *cy = k & 1 ? yb : ya;
                 double *tx = k & 1 ? xa : xb, *ty = k & 1 ? ya : yb;
                 bool ch = false;
                 for (int t = tid; t < nw; t += kFimThreads) {
                     const int q = work[t], lx = q % REG, ly = q / REG;
-                    if (lx < ring || lx >= REG - ring || ly < ring || ly >= REG - ring) continue;
-                    const double pp = ph[q];
-                    double acc[6] = {0, 0, 0, 0, 0, 0}, c[3];
-                    if (k == 0) {
-                        ExtFit f;
-                        f.clear();
-#pragma unroll
-                        for (int dj = -3; dj <= 3; dj++)
-#pragma unroll
-                            for (int di = -3; di <= 3; di++) {
-                                const int e = q + dj * REG + di;
-                                const double p = ph[e];
-                                if (!(p < pp)) continue;
-                                const double ww = pp - p;
-                                f.moments(di, dj, ww);
-                                ExtFit::values(di, dj, ww, cx[e], cy[e], acc);
-                            }
-                        const double det = f.det();
-                        if (fabs(det) < 1e-10) flags[11] = 1;
-                        f.solve(det, c);
-                        fit[t] = c[0];
-                        fit[NL + t] = c[1];
-                        fit[2 * NL + t] = c[2];
+                    if (!WIDE && (lx < ring || lx >= REG - ring || ly < ring || ly >= REG - ring)) continue;
+                    double ox, oy;
+                    if constexpr (WIDE) {
+                        if (!ext_widen(ph, cx, cy, q, REG, ox, oy)) {
+                            flags[5] = INCRMT_ERR_EXTRAP_SINGULAR;
+                            ox = cx[q];
+                            oy = cy[q];
+                        }
                     } else {
-#pragma unroll 1
-                        for (int dj = -3; dj <= 3; dj++)
+                        const double pp = ph[q];
+                        double acc[6] = {0, 0, 0, 0, 0, 0}, c[3];
+                        if (k == 0) {
+                            ExtFit f;
+                            f.clear();
 #pragma unroll
-                            for (int di = -3; di <= 3; di++) {
-                                const int e = q + dj * REG + di;
-                                const double p = ph[e];
-                                if (!(p < pp)) continue;
-                                ExtFit::values(di, dj, pp - p, cx[e], cy[e], acc);
-                            }
-                        c[0] = fit[t]; c[1] = fit[NL + t]; c[2] = fit[2 * NL + t];
+                            for (int dj = -3; dj <= 3; dj++)
+#pragma unroll
+                                for (int di = -3; di <= 3; di++) {
+                                    const int e = q + dj * REG + di;
+                                    const double p = ph[e];
+                                    if (!(p < pp)) continue;
+                                    const double ww = pp - p;
+                                    f.moments(di, dj, ww);
+                                    ExtFit::values(di, dj, ww, cx[e], cy[e], acc);
+                                }
+                            const double det = f.det();
+                            if (ExtFit::singular(det)) flags[11] = 1;
+                            f.solve(det, c);
+                            fit[t] = c[0];
+                            fit[NL + t] = c[1];
+                            fit[2 * NL + t] = c[2];
+                        } else {
+#pragma unroll 1
+                            for (int dj = -3; dj <= 3; dj++)
+#pragma unroll
+                                for (int di = -3; di <= 3; di++) {
+                                    const int e = q + dj * REG + di;
+                                    const double p = ph[e];
+                                    if (!(p < pp)) continue;
+                                    ExtFit::values(di, dj, pp - p, cx[e], cy[e], acc);
+                                }
+                            c[0] = fit[t]; c[1] = fit[NL + t]; c[2] = fit[2 * NL + t];
+                        }
+                        ox = ExtFit::value(acc, c);
+                        oy = ExtFit::value(acc + 3, c);
                     }
-                    const double ox = ExtFit::value(acc, c), oy = ExtFit::value(acc + 3, c);
                     if ((ox != cx[q] || oy != cy[q]) && lx >= E::kHalo && lx < E::kHalo + TILE && ly >= E::kHalo &&
                         ly < E::kHalo + TILE)
                         ch = true;
@@ -1028,23 +961,54 @@ __global__ void __launch_bounds__(kFimThreads, 1) k_ls_extrap_tiles(LsGrid g, co
             for (int t = tid; t < nw; t += kFimThreads) {
                 const int q = work[t], lx = q % REG, ly = q / REG, i = x0 + lx, j = y0 + ly;
                 if (lx >= E::kHalo && lx < E::kHalo + TILE && ly >= E::kHalo && ly < E::kHalo + TILE && i < xe && j < ye) {
-                    ox[j * g.P + i] = SWEEPS & 1 ? xb[q] : xa[q];
-                    oy[j * g.P + i] = SWEEPS & 1 ? yb[q] : ya[q];
+                    ox[j * g.P + i] = xb[q];
+                    oy[j * g.P + i] = yb[q];
                 }
             }
         }
         grid.sync();
-        if (*reinterpret_cast<volatile int *>(&flags[11])) break;
+        // (a singular fit depends on the level set alone: the first batch raises
+        // its flag or none does)
+        if (*reinterpret_cast<volatile int *>(&flags[WIDE ? 5 : 11])) return -1;
         const int mask = *reinterpret_cast<volatile int *>(&flags[batch % 3]);
         const int last = __ffs(~mask) - 1;  // the first sweep that changed nothing
-        if (last < SWEEPS && it0 + last < max_sweeps) {
-            it0 += last + 1;
-            done = true;
-            break;
-        }
+        if (last < kRun && it0 + last < max_sweeps) return it0 + last + 1;
     }
-    if (blockIdx.x == 0 && tid == 0) { flags[3] = done ? it0 : max_sweeps; flags[4] = done ? 1 : 0; }
+    return -1;
 }
+
+/** All sweeps of the extrapolation wavefront in one cooperative launch, staged
+ * like the march (k_ls_fim_coop): the fit's moments depend on the level set
+ * alone and are formed by the first sweep of a batch; the others only sum the
+ * values of the 7 x 7 window. The first batch reads the reference map itself. A
+ * point whose window of radius 3 gives a singular fit (a grid in small units,
+ * where the weights are small) raises flags[11] and ends the launch after its
+ * first batch; a WIDE launch then starts over from batch 1 with one sweep per
+ * batch, for which the halo holds the widest window, and a fit that stays
+ * singular raises flags[5]. (One launch for both took the usual batches 1 to 5
+ * per cent longer, for the registers.) flags[0..2], [3] and [4] as in
+ * k_ls_fim_coop; the values are in o.b, o.d if the last batch's number is even
+ * (ext_in_b).
+ *
+ * Bound by the window sums of the busiest SM. Measured (B200, us per call, one
+ * sweep per barrier over global memory -> here): rotor 128^2 266 -> 108, 1024^2
+ * 288 -> 107; 32 bodies 1024 x 2048 377 -> 271; flag 2048^2 469 -> 211. Both
+ * launches of a circle with windows of radius 4, 22 sweeps: 256^2 940 -> 524,
+ * 1024^2 1245 -> 531. */
+template <int TILE, int SWEEPS, bool WIDE>
+__global__ void __launch_bounds__(kFimThreads, 1) k_ls_extrap_tiles(LsGrid g, const LsObj *ob, const LsWin *win, const int *list,
+                                                                    const int *list_k, const int *countp, int cap, int *flags,
+                                                                    int max_sweeps) {
+    const int sweeps = ext_batches<TILE, SWEEPS, WIDE>(g, ob, win, list, list_k, min(*countp, cap), flags, max_sweeps);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        flags[3] = sweeps < 0 ? max_sweeps : sweeps;
+        flags[4] = sweeps >= 0;
+    }
+}
+
+/** Whether k_ls_extrap_tiles left its values in o.b, o.d: its batches are the
+ * sweeps in groups, or a first batch given up and then one per sweep. */
+inline bool ext_in_b(int sweeps, int per_batch, bool wide) { return (wide ? sweeps + 1 : cdiv(sweeps, per_batch)) & 1; }
 
 /** Stores the values of k_ls_extrap_tiles (in o.b, o.d if in_b) into nX, nY. */
 __global__ void k_ls_extrap_keep(LsGrid g, const LsObj *ob, const LsWin *win, bool in_b) {
@@ -1055,43 +1019,6 @@ __global__ void k_ls_extrap_keep(LsGrid g, const LsObj *ob, const LsWin *win, bo
     if (!ls_outside(o.s[ij])) return;
     o.nX[ij] = in_b ? o.b[ij] : o.a[ij];
     o.nY[ij] = in_b ? o.d[ij] : o.c[ij];
-}
-
-/** All sweeps of the extrapolation wavefront over global memory in one
- * cooperative launch, each followed by a grid barrier, for fits that need a
- * window wider than radius 3; flags[5] is raised where it stays singular. */
-__global__ void __launch_bounds__(kExtrapThreads, 1) k_ls_extrap_coop(LsGrid g, const LsObj *ob, const int *list, const int *list_k,
-                                 const int *countp, int cap, int *flags, int max_sweeps) {
-    namespace cg = cooperative_groups;
-    cg::grid_group grid = cg::this_grid();
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
-    const int count = min(*countp, cap);
-    int it = 0;
-    bool done = false;
-    for (; it < max_sweeps; it++) {
-        if (tid == 0) flags[(it + 1) % 3] = 0;
-        const bool odd = it & 1;
-        bool ch = false;
-        for (int t = tid; t < count; t += nth) {
-            const LsObj &o = ob[list_k[t]];
-            const double *cx = odd ? o.b : o.a, *cy = odd ? o.d : o.c;
-            double *tx = odd ? o.a : o.b, *ty = odd ? o.c : o.d;
-            const int ij = list[t], i = ij % g.P, j = ij / g.P;
-            double ox, oy;
-            if (!ls_extrap_point(g, o.s, o.phi, o.nX, o.nY, cx, cy, i, j, ox, oy)) {
-                atomicExch(&flags[5], INCRMT_ERR_EXTRAP_SINGULAR);
-                ox = cx[ij]; oy = cy[ij];
-            }
-            if (ox != cx[ij] || oy != cy[ij]) ch = true;
-            tx[ij] = ox;
-            ty[ij] = oy;
-        }
-        if (__syncthreads_or(ch) && threadIdx.x == 0) flags[it % 3] = 1;
-        grid.sync();
-        const int c = *reinterpret_cast<volatile int *>(&flags[it % 3]);
-        if (!c) { done = true; break; }
-    }
-    if (tid == 0) { flags[3] = done ? it + 1 : it; flags[4] = done ? 1 : 0; }
 }
 
 }  // namespace incrmt

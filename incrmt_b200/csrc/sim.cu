@@ -49,10 +49,10 @@ struct Sim {
     double *src_mac = nullptr, *z_mac = nullptr, *src_fem = nullptr, *z_fem = nullptr;
     std::vector<LsObj> lso;                         // level-set working arrays per object
     LsObj *d_lso = nullptr;
-    int *d_list = nullptr, *d_list_k = nullptr;     // combined point list of all objects
+    int *d_list = nullptr, *d_list_k = nullptr;     // combined tile list of all objects
     int list_cap = 0;
     std::vector<void *> raw_allocs;                 // non-double per-object arrays
-    int coop_blocks_fim = 0, coop_blocks_ext = 0;   // co-resident grid sizes
+    int coop_blocks_fim = 0;                        // co-resident grid size
     int *d_flags = nullptr;  // [0..2] sweep change flags, [3] sweeps, [4] converged, [5] fit error,
                            // [6] Newton error, [7] list length, [8] tracer remaps, [9] correction failure
     int *h_flags = nullptr;                         // pinned
@@ -315,16 +315,19 @@ int Sim::create(const incrmt_grid *gr, const incrmt_phys *ph) {
                                        static_cast<int>(Fim<kFimSmall, kFimSweeps>::kSmem)));
         INCRMT_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fim, kFimThreads, fsm));
         coop_blocks_fim = sms * (nb > 0 ? 1 : 0);
-        const auto ext = k_ls_extrap_tiles<kFimLarge, kExtSweeps>;
-        constexpr size_t esm = Ext<kFimLarge, kExtSweeps>::kSmem;
-        INCRMT_CK(cudaFuncSetAttribute(ext, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(esm)));
-        INCRMT_CK(cudaFuncSetAttribute(k_ls_extrap_tiles<kFimSmall, kExtSweeps>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(Ext<kFimSmall, kExtSweeps>::kSmem)));
-        INCRMT_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ext, kFimThreads, esm));
+        constexpr size_t esm = Ext<kFimLarge, kExtSweeps>::kSmem, ess = Ext<kFimSmall, kExtSweeps>::kSmem;
+        const auto attr = [](auto k, size_t b) {
+            return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(b));
+        };
+        INCRMT_CK(attr(k_ls_extrap_tiles<kFimLarge, kExtSweeps, false>, esm));
+        INCRMT_CK(attr(k_ls_extrap_tiles<kFimLarge, kExtSweeps, true>, esm));
+        INCRMT_CK(attr(k_ls_extrap_tiles<kFimSmall, kExtSweeps, false>, ess));
+        INCRMT_CK(attr(k_ls_extrap_tiles<kFimSmall, kExtSweeps, true>, ess));
+        INCRMT_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_ls_extrap_tiles<kFimLarge, kExtSweeps, false>, kFimThreads, esm));
         if (nb == 0) coop_blocks_fim = 0;
-        INCRMT_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_ls_extrap_coop, kExtrapThreads, 0));
-        coop_blocks_ext = sms * (nb > 0 ? 1 : 0);
-        if (coop_blocks_fim == 0 || coop_blocks_ext == 0) {
+        INCRMT_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_ls_extrap_tiles<kFimLarge, kExtSweeps, true>, kFimThreads, esm));
+        if (nb == 0) coop_blocks_fim = 0;
+        if (coop_blocks_fim == 0) {
             set_error("level-set kernels cannot be co-resident");
             return INCRMT_ERR_CUDA;
         }
@@ -485,10 +488,10 @@ int Sim::upload_objects() {
     INCRMT_CK(cudaMemcpyAsync(d_obj, obj.data(), sizeof(ObjDev) * obj.size(), cudaMemcpyHostToDevice, stream));
     INCRMT_CK(cudaMemcpyAsync(d_sol, sol.data(), sizeof(SolidDev) * sol.size(), cudaMemcpyHostToDevice, stream));
     INCRMT_CK(cudaMemcpyAsync(d_lso, lso.data(), sizeof(LsObj) * lso.size(), cudaMemcpyHostToDevice, stream));
-    // Room for every point of every object in the combined level-set list.
+    // The combined tile list: room for every point of every object.
     const size_t need = cells() * obj.size();
     if (need > static_cast<size_t>(list_cap)) {
-        if (need > 0x7fffffffu) { set_error("level-set point list too large"); return INCRMT_ERR_BADARG; }
+        if (need > 0x7fffffffu) { set_error("level-set list too large"); return INCRMT_ERR_BADARG; }
         cudaFree(d_list);
         cudaFree(d_list_k);
         d_list = d_list_k = nullptr;
@@ -729,8 +732,7 @@ int Sim::pin() {
 }
 
 /** levelset::extrapolate_fields for every object (traverse.hh:235-260),
- * the objects' wavefronts settling together in one cooperative launch: in
- * staged tiles, or (a fit that needs a wider window) over global memory. */
+ * the objects' wavefronts settling together in one cooperative launch. */
 int Sim::extrapolate_all() {
     const int no = static_cast<int>(obj.size());
     if (no == 0) return INCRMT_OK;
@@ -752,35 +754,28 @@ int Sim::extrapolate_all() {
     launches++;
     INCRMT_CKL("collect");
     void *targs[] = {&lg, &ob, &wl, &d_list, &d_list_k, &countp, &cap, &d_flags, &maxs};
-    INCRMT_CK(cudaLaunchCooperativeKernel(small ? reinterpret_cast<void *>(k_ls_extrap_tiles<kFimSmall, kExtSweeps>)
-                                                : reinterpret_cast<void *>(k_ls_extrap_tiles<kFimLarge, kExtSweeps>),
-                                          dim3(coop_blocks_fim), dim3(kFimThreads), targs,
-                                          small ? Ext<kFimSmall, kExtSweeps>::kSmem : Ext<kFimLarge, kExtSweeps>::kSmem, stream));
-    launches++;
+    const auto launch = [&](void *tiles_small, void *tiles_large) {
+        launches++;
+        return cudaLaunchCooperativeKernel(small ? tiles_small : tiles_large, dim3(coop_blocks_fim), dim3(kFimThreads), targs,
+                                           small ? Ext<kFimSmall, kExtSweeps>::kSmem : Ext<kFimLarge, kExtSweeps>::kSmem, stream);
+    };
+    INCRMT_CK(launch(reinterpret_cast<void *>(k_ls_extrap_tiles<kFimSmall, kExtSweeps, false>),
+                     reinterpret_cast<void *>(k_ls_extrap_tiles<kFimLarge, kExtSweeps, false>)));
     int r = fetch_flags();
     if (r) return r;
     const bool wide = h_flags[11] != 0;
     if (wide) {
-        INCRMT_CK(cudaMemsetAsync(d_flags, 0, sizeof(int) * 12, stream));
-        k_ls_collect_outside<<<gg, kB2, 0, stream>>>(lg, d_lso, wl, d_list, d_list_k, d_flags + 7, list_cap, d_flags + 10);
-        k_ls_extrap_init<<<4 * kB200SMs, 256, 0, stream>>>(d_lso, d_list, d_list_k, d_flags + 7, list_cap);
-        launches += 2;
-        INCRMT_CKL("collect");
-        void *args[] = {&lg, &ob, &d_list, &d_list_k, &countp, &cap, &d_flags, &maxs};
-        INCRMT_CK(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(k_ls_extrap_coop), dim3(coop_blocks_ext),
-                                              dim3(kExtrapThreads), args, 0, stream));
-        launches++;
+        INCRMT_CK(launch(reinterpret_cast<void *>(k_ls_extrap_tiles<kFimSmall, kExtSweeps, true>),
+                         reinterpret_cast<void *>(k_ls_extrap_tiles<kFimLarge, kExtSweeps, true>)));
         if ((r = fetch_flags())) return r;
     }
     if (h_flags[5]) { set_error("singular extrapolation fit"); return h_flags[5]; }
     if (h_flags[10]) { set_error("extrapolation list overflow"); return INCRMT_ERR_BADARG; }
     ex_sweeps += h_flags[3];
     if (!h_flags[4]) { set_error("extrapolation did not settle in %d sweeps", h_flags[3]); return INCRMT_ERR_NOCONV; }
-    // After the last sweep both buffers hold the same values.
-    if (wide) k_ls_extrap_store<<<4 * kB200SMs, 256, 0, stream>>>(d_lso, d_list, d_list_k, d_flags + 7, list_cap);
-    else k_ls_extrap_keep<<<gg, kB2, 0, stream>>>(lg, d_lso, wl, cdiv(h_flags[3], kExtSweeps) & 1);
+    k_ls_extrap_keep<<<gg, kB2, 0, stream>>>(lg, d_lso, wl, ext_in_b(h_flags[3], kExtSweeps, wide));
     launches++;
-    INCRMT_CKL("k_ls_extrap_store");
+    INCRMT_CKL("k_ls_extrap_keep");
     return INCRMT_OK;
 }
 

@@ -56,7 +56,8 @@ def fit(phi, band, X, Y, j, i, r):
 
 
 def extrapolated(m, n, L, shape):
-    """phi, status and the reference map of a bent body after one extrapolation."""
+    """phi, status and the reference map of a bent body after one extrapolation;
+    no map where it reports a singular fit."""
     from incrmt_b200 import capi
     s = capi.Simulation(m, n, ax=-L, bx=L, ay=-L, by=L, visc=1e-2 * L * L, ntrace=0)
     SHAPES[shape](s, L)
@@ -64,7 +65,11 @@ def extrapolated(m, n, L, shape):
     X, Y = s.get("X"), s.get("Y")
     s.set("nX", X + 0.01 * L * np.sin(3 * Y / L))
     s.set("nY", Y + 0.02 * L * np.cos(2 * X / L))
-    s.stage("extrapolate")
+    try:
+        s.stage("extrapolate")
+    except capi.IncrmtError as e:
+        assert e.code == capi.ERR_EXTRAP_SINGULAR
+        return s, s.get("phi"), s.get("status"), None, None
     return s, s.get("phi"), s.get("status"), s.get("nX"), s.get("nY")
 
 
@@ -79,4 +84,35 @@ def test_regular_fits_to_the_bit(gpu, shape, m, n):
         det, x, y = fit(phi, band, X, Y, j, i, 3)
         assert abs(det) >= 1e-10
         assert x == X[j, i] and y == Y[j, i], (j, i)
+    s.close()
+
+
+@pytest.mark.parametrize("shape", list(SHAPES))
+@pytest.mark.parametrize("m,L,radius", [
+    (64, 3.2e-4, 4),     # some radius-3 fits are singular, some are not
+    (64, 2.5e-4, 4),
+    (64, 1.2e-4, 5),
+    (256, 1e-3, 4),      # many tiles
+])
+def test_singular_fits_widen(gpu, shape, m, L, radius):
+    """A grid in small units: its weights are so small that the determinant falls
+    below the singular limit at radius 3, and not at a wider one."""
+    s, phi, st, X, Y = extrapolated(m, m, L, shape)
+    band = (st >= 2) & (st <= 5)
+    points = np.argwhere((st == 4) | (st == 5))
+    if X is None:  # reported only where a fit is singular at every radius (bands cut by the grid's edge)
+        assert any(all(abs(fit(phi, band, phi, phi, j, i, r)[0]) < 1e-10 for r in range(3, 8)) for j, i in points)
+        s.close()
+        return
+    widest = 0
+    for j, i in points[::max(len(points) // 60, 1)]:
+        r = 3
+        while r < 8:
+            det, x, y = fit(phi, band, X, Y, j, i, r)
+            if abs(det) >= 1e-10:
+                break
+            r += 1
+        widest = max(widest, r)
+        assert x == X[j, i] and y == Y[j, i], (j, i, r)
+    assert widest >= radius
     s.close()
