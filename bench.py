@@ -713,7 +713,8 @@ def run_ours_sim(args, ws, rank, local, dist):
     roof = _roofline(f"{args.workload}_smooth", sm_ms, sm_bytes, sm_launch,
                      "k_smooth_cells on the fine level of the MAC and FEM projections "
                      "(two Gauss-Seidel sweeps per launch)",
-                     "updated unknowns x 2 sweeps x (3+c) x w; c=2 MAC, 1 FEM")
+                     "unknowns x (3+c) x w, operands and result once for both sweeps (from zero: one word fewer); "
+                     "c=2 MAC, 1 FEM")
     if roof is not None:
         roof["projection"] = projection_roofline(None, args.workload, prec, a["vc_mac"], a["vc_fem"], a["phases"])
         if plain is not None and "phases" in plain:
@@ -988,7 +989,7 @@ def run_ours(args, ws, rank, local, dist):
         "vcycles_per_projection": float(np.mean(vcs)),
         "roofline": _roofline("mac4096_smooth", kms, kbytes, klaunch,
                               "k_smooth_cells (fine-level Gauss-Seidel, two sweeps per launch)",
-                              "updated unknowns x 2 sweeps x (3+c) x w, c=2 (MAC)"),
+                              "unknowns x (3+c) x w, operands and result once for both sweeps, c=2 (MAC)"),
         "cpu_baseline": cpu,
         "e2e": {"value": e2e, "unit": "steps/s",
                 "h2d_bytes_per_step": h2d_bytes, "d2h_bytes_per_step": d2h_bytes},

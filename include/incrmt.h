@@ -150,8 +150,9 @@ long long incrmt_mg_mixed_fallbacks(const incrmt_mg *h);
 long long incrmt_mg_coarse_builds(const incrmt_mg *h, long long *retries);
 
 /** Accumulated profile since incrmt_mg_set_profiling: total device time (ms)
- * of the timed launches, their algorithmic bytes (updated unknowns x (3+c)
- * words) and their number. */
+ * of the timed launches, the bytes they cannot do without (operands read and
+ * results written once: (3+c) words an unknown, c = 2 MAC or 1 FEM, one fewer
+ * from a zero start) and their number. */
 int incrmt_mg_profile(incrmt_mg *h, double *ms, double *bytes, long long *launches);
 
 /** The handle's CUDA stream (a cudaStream_t), on which every kernel and copy

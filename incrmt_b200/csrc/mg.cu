@@ -831,15 +831,15 @@ cudaError_t set_tail_attr() {
  * reads z and writes zalt (*res = zalt); otherwise one launch per colour
  * updates z in place (*res = z). zero: the sweeps start from 0 and z need not
  * hold it (tiles then read no iterate). When prof is given, each launch is bracketed
- * by CUDA events and credited with its algorithmic bytes: (units updated) x
- * bytes_per_unit. */
+ * by CUDA events and credited with the bytes it cannot do without: its operands
+ * read and its result written once, bytes_per_unit for each unknown it updates. */
 template <class Op, class T>
 int smooth(Op op, T *z, T *zalt, const T *b, int m, int n, int sweeps, cudaStream_t s, long long &nl, T **res,
            bool zero = false, Multigrid *prof = nullptr, double bytes_per_unit = 0) {
     *res = z;
     if (sweeps == 2 && zalt && (!op.px || m % 2 == 0) && (!op.py || n % 2 == 0)) {
         const double words = zero ? sizeof(T) : 0;  // not read
-        if (prof) { int r = prof->prof_begin(static_cast<double>(m) * n * (2 * bytes_per_unit - words)); if (r) return r; }
+        if (prof) { int r = prof->prof_begin(static_cast<double>(m) * n * (bytes_per_unit - words)); if (r) return r; }
         smooth_cells(op, zero ? static_cast<const T *>(nullptr) : z, zalt, b, m, n, s);
         nl++;
         if (prof) { int r = prof->prof_end(); if (r) return r; }
@@ -1245,8 +1245,8 @@ int Multigrid::cycle64(int l, const double *b0, double *z0, bool zero) {
     const MgLevel &C = lev[l + 1];
     int r;
     Multigrid *pf = prof ? this : nullptr;
-    // Algorithmic bytes per updated unknown of a fine FP64 sweep: read z,b
-    // and the coefficient words, write z (3+c words; c=2 MAC, c=1 FEM).
+    // Bytes per unknown of a fine FP64 smoothing launch: read z, b and the
+    // coefficient words, write z (3+c words; c=2 MAC, c=1 FEM).
     const double bpu = 8.0 * (sys == INCRMT_SYS_MAC ? 5 : 4);
     // Pre-smoothing may leave the iterate in the level's second buffer; the
     // restriction, prolongation and post-smoothing follow it, and the
