@@ -136,24 +136,27 @@ def _traffic(key):
         return json.load(f).get(key)
 
 
-def vcycle_pass_bytes(m, n, c0, w=8, tail=1024):
+def vcycle_pass_bytes(m, n, c0, w=8, tail=128 * 128):
     """Compulsory bytes of one FP64 V-cycle as the kernels run it on an
     isotropic grid (standard coarsening): on a level of N unknowns with c
     coefficient words each (c0 on the fine level, 9 on the Galerkin levels),
     two tile-fused smoothing launches read z, b and the coefficients and write
-    z ((3 + c) words each), the restriction reads z, b, the coefficients and
-    four prolongation weights (6 + c) and writes b and z of the coarse level,
-    the prolongation reads the weights and z and writes z (6) and reads each
-    coarse value once: (18 + 3c) N + 3 N_coarse words; the fine level adds the
-    residual norm (2 + c) N. Levels of at most `tail` unknowns run in one
-    block from shared memory and are not counted."""
+    z ((3 + c) words each; on a coarse level the first starts from zero and
+    reads no z), the restriction reads z, b, the coefficients and two
+    prolongation weights (4 + c) and writes the coarse b, the prolongation
+    reads the weights and z and writes z (4) and reads each coarse value once:
+    (14 + 3c) N + 2 N_coarse words, N fewer on a coarse level; the fine level
+    adds the residual norm (2 + c) N. Levels of at most `tail` unknowns run in
+    one cluster on chip and are not counted."""
     total, c, first = 0.0, c0, True
     while m * n > tail:
         mc, nc = (m + 1) // 2, (n + 1) // 2
-        total += (18 + 3 * c) * m * n + 3 * mc * nc
+        total += (14 + 3 * c) * m * n + 2 * mc * nc
         if first:
             total += (2 + c) * m * n
             first = False
+        else:
+            total -= m * n
         m, n, c = mc, nc, 9
     return total * w
 
@@ -1020,9 +1023,9 @@ def run_ours(args, ws, rank, local, dist):
                 "achieved": ach2, "peak": peak, "unit": "GB/s", "frac": ach2 / peak, "peak_kind": kind,
                 "bytes_per_vcycle": pb, "time": "whole step including the density setup",
                 "bytes_rule": "per level of N unknowns with c coefficient words (2 fine MAC, 9 Galerkin): "
-                              "(18 + 3c) N w for two smoothing launches, the restriction and the prolongation "
-                              "as implemented (each reading its arrays once), 3 w per coarse unknown, and the "
-                              "fine residual norm (2 + c) N w"}
+                              "(14 + 3c) N w for two smoothing launches, the restriction and the prolongation "
+                              "as implemented (each reading its arrays once; N w fewer on coarse levels, which "
+                              "start from zero), 2 w per coarse unknown, and the fine residual norm (2 + c) N w"}
     print(json.dumps(line))
     release()
 

@@ -157,8 +157,10 @@ constexpr int kGalRows = 4;  // coarse rows of a tile
  * Bound by the sums' shared-memory reads and FP64 latency. Four rows leave room
  * for three blocks per SM, and the sums have no branches: a point's zero
  * weights are known from its parities. Measured (B200, us; 8 rows, tests of
- * every weight -> here): MAC 4096^2 1782 -> 848 (8 rows 1163, 2 rows 1044), the
- * 2048^2 flag's Galerkin levels 42.1 -> 18.7, FEM 1024^2 152 -> 57. */
+ * every weight -> here): MAC 4096^2 1782 -> 920 (8 rows 1163, 2 rows 1044), the
+ * 2048^2 flag's Galerkin levels 42.1 -> 20.1. Staging the weights from the planes
+ * takes 7 to 8% longer here than from an array with four per point, whose
+ * writing took k_build_p as long again. */
 template <class Op, bool KX, bool KY>
 __global__ void __launch_bounds__(32 * kGalRows) k_galerkin_tile(Op op, int fm, int fn, int px, int py, int cm, int cn,
                                                        double *st, const double *Q) {

@@ -11,11 +11,13 @@
 // (40 doubles of stencil and right-hand side per thread: 512 threads; four cell
 // densities in FEM or edges in MAC shared between a cell's points: 1024).
 //
-// Large levels are bound by L2 traffic (the tile with its halo) and, FEM and
-// MAC in double, by the divisions; small ones by one load latency and eight
-// phases, 4 to 5 us. Measured (B200, two sweeps, us; the former kernels first:
-// a pipeline along y for the large fine levels, a 64 x 32 or 32 x 16 tile of
-// unknowns that read its coefficients from L2 in every phase otherwise):
+// Large MAC levels in double are bound by L1 and shared memory (75% busy, DRAM at
+// 39%, loads the first stall), the single-precision ones by issue (53 to 60%),
+// Galerkin levels in double by the phases' latency (one block of 16 warps per
+// SM); small levels by one load latency and eight phases, 4 to 5 us. Measured
+// (B200, two sweeps, us; the former kernels first: a pipeline along y for the
+// large fine levels, a 64 x 32 or 32 x 16 tile of unknowns that read its
+// coefficients from L2 in every phase otherwise):
 //
 //                MAC                 FEM                 Galerkin
 //   size      FP64      FP32      FP64      FP32      FP64      FP32
@@ -328,7 +330,8 @@ void smooth_cells_launch(bool pair, const Op &op, const T *z, T *zout, const T *
  *
  * Tile heights, from sweeps over 10 to 32: MAC 16 (FP64 4096^2: 12 rows 194,
  * 16 rows 173, 32 rows 188 us); Galerkin 16 (FP64 2048^2: 14 rows 180, 16 rows
- * 160, 18 rows, spilling, 161). FEM: the tallest that fits (FP64 4096^2: 16 rows
+ * 160, 18 rows, spilling, 161; FP32, mean of a 4096^2 MAC system's four levels: 12
+ * rows 41, 16 rows, two blocks per SM, 27, 24 rows, one block, 33). FEM: the tallest that fits (FP64 4096^2: 16 rows
  * 464, 24 rows 331, 32 rows 281; FP32: 16 rows 190, 24 rows 170), except where
  * 16 rows make a grid that all runs at once: fewer warps per tile then shorten
  * the phases (FP64 257^2: 16 rows 6.0, 32 rows 11.3; FP32 513^2: 16 rows 8.8, 24

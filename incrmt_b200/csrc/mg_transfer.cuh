@@ -35,9 +35,10 @@ constexpr int kPX = 32, kPY = 8;  // cells of a block of k_build_p
  *
  * One thread per cell; where both directions are halved the blocks overlap by
  * a column and a row, whose cells' edge weights the last points need. Bound by
- * the loads' latency and the quotients. Measured (B200, us, two passes of one
- * thread per point -> here): MAC 4096^2 613 -> 251, its Galerkin levels 37 -> 14
- * each, FEM 1024^2 55 -> 17. */
+ * the loads' latency and, on the fine level, by memory (4.1 TB/s). Measured (B200,
+ * us, two passes of one thread per point -> here): MAC 4096^2 613 -> 124, its
+ * Galerkin levels 37 -> 9 each (251 and 14 while it wrote four weights per point
+ * as well). */
 template <class Op, bool KX, bool KY>
 __global__ void __launch_bounds__(kPX * kPY) k_build_p(Op op, int fm, int fn, int px, int py, int cm, int cn, double *Q) {
     constexpr bool both = KX && KY;
