@@ -157,10 +157,10 @@ constexpr int kGalRows = 4;  // coarse rows of a tile
  * Bound by the sums' shared-memory reads and FP64 latency. Four rows leave room
  * for three blocks per SM, and the sums have no branches: a point's zero
  * weights are known from its parities. Measured (B200, us; 8 rows, tests of
- * every weight -> here): MAC 4096^2 1782 -> 920 (8 rows 1163, 2 rows 1044), the
- * 2048^2 flag's Galerkin levels 42.1 -> 20.1. Staging the weights from the planes
- * takes 7 to 8% longer here than from an array with four per point, whose
- * writing took k_build_p as long again. */
+ * every weight -> here): MAC 4096^2 1782 -> 660 (8 rows 1163, 2 rows 1044), the
+ * 2048^2 flag's Galerkin levels 42.1 -> 15.5, FEM 1024 x 2048 94. Weights staged by
+ * points take 920 from the planes and 850 from an array with four per point
+ * (4096^2). */
 template <class Op, bool KX, bool KY>
 __global__ void __launch_bounds__(32 * kGalRows) k_galerkin_tile(Op op, int fm, int fn, int px, int py, int cm, int cn,
                                                        double *st, const double *Q) {
@@ -174,23 +174,46 @@ __global__ void __launch_bounds__(32 * kGalRows) k_galerkin_tile(Op op, int fm, 
     const int X0 = blockIdx.x * CTW, Y0 = blockIdx.y * CTH;
     const int SX0 = kx ? 2 * X0 - 1 : X0, SY0 = ky ? 2 * Y0 - 1 : Y0;
     constexpr int SW = kx ? 2 * CTW + 1 : CTW, SH = ky ? 2 * CTH + 1 : CTH, SA = SW * SH;
-    const int NX0 = SX0 - 1, NY0 = SY0 - 1;
     constexpr int NW = SW + 2, NH = SH + 2;
-    double *As = gal_smem;          // entry k of support point t at As[k * SA + t]
-    double *Ps = gal_smem + 9 * SA;  // weights of region point t at Ps[4 * t .. 4 * t + 3]
+    double *Ps = gal_smem;             // weights of region point t at Ps[4 * t .. 4 * t + 3]
+    double *As = Ps + 4 * (NW * NH);  // entry k of support point t at As[k * SA + t]
     // Only the supports of coarse points I < cm, J < cn (fine x up to sxmax)
     // and their stencil neighbours (one further) are read below. Beyond them
     // the region of a level smaller than the tile would reach more than one
     // period past a periodic grid, where one wrap does not bring an index
     // back inside it: such points are not staged.
     const int sxmax = kx ? 2 * cm - 1 : cm - 1, symax = ky ? 2 * cn - 1 : cn - 1;
-    for (int t = threadIdx.x; t < NW * NH; t += blockDim.x) {
-        const int xu = NX0 + t % NW, yu = NY0 + t / NW;
-        bool ok = xu <= sxmax + 1 && yu <= symax + 1;
-        const int i = wrap_idx(xu, fm, px, ok), j = wrap_idx(yu, fn, py, ok);
-        double w[4] = {0, 0, 0, 0};
-        if (ok) plane_weights(Q, cells_of(fm, kx), cells_of(fn, ky), kx, ky, i, j, w);
-        Ps[4 * t] = w[0]; Ps[4 * t + 1] = w[1]; Ps[4 * t + 2] = w[2]; Ps[4 * t + 3] = w[3];
+    // The weights by cells (the region starts on one; a periodic direction has
+    // whole ones): all of a cell's planes are loaded together.
+    constexpr int CW = KX ? (NW + 1) / 2 : NW, CH = KY ? (NH + 1) / 2 : NH;
+    const int cx = cells_of(fm, kx), cy = cells_of(fn, ky);
+    const long NC = static_cast<long>(cx) * cy;
+    for (int t = threadIdx.x; t < CW * CH; t += blockDim.x) {
+        const int a = t % CW, b = t / CW, Iu = X0 - 1 + a, Ju = Y0 - 1 + b;
+        bool ok = (kx ? 2 * Iu : Iu) <= sxmax + 1 && (ky ? 2 * Ju : Ju) <= symax + 1;
+        const int I = wrap_idx(Iu, cx, px, ok), J = wrap_idx(Ju, cy, py, ok);
+        constexpr int kPlanes = KX && KY ? 8 : 2;
+        double w[kPlanes];
+        const double *q = Q + I + static_cast<long>(cx) * J;
+#pragma unroll
+        for (int e = 0; e < kPlanes; e++) w[e] = ok ? q[e * NC] : 0.0;
+        auto put = [&](int u, int v, double w0, double w1, double w2, double w3) {
+            const int x = kx ? 2 * a + u : a, y = ky ? 2 * b + v : b;
+            if (x >= NW || y >= NH) return;
+            double2 *p = reinterpret_cast<double2 *>(Ps + 4 * (x + NW * y));
+            p[0] = make_double2(w0, w1);
+            p[1] = make_double2(w2, w3);
+        };
+        put(0, 0, ok ? 1.0 : 0.0, 0, 0, 0);
+        if constexpr (KX && KY) {
+            put(1, 0, w[0], w[1], 0, 0);
+            put(0, 1, w[2], 0, w[3], 0);
+            put(1, 1, w[4], w[5], w[6], w[7]);
+        } else if constexpr (KX) {
+            put(1, 0, w[0], w[1], 0, 0);
+        } else {
+            put(0, 1, w[0], 0, w[1], 0);
+        }
     }
     for (int t = threadIdx.x; t < SA; t += blockDim.x) {
         const int xu = SX0 + t % SW, yu = SY0 + t / SW;

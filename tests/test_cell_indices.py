@@ -124,7 +124,35 @@ def test_galerkin_tiles(grid, monkeypatch):
             continue  # an index is wrapped once: only levels of about a tile can need it twice
         if fm * fn > 60000:
             continue
+        # the supports' stencils are staged by points
         assert tiles.replay_galerkin(fm, fn, cm, cn, kx, ky, px, py) == (0, 0)
+        # the weights by cells, each direction by itself
+        for f, c, k, p, width in ((fm, cm, kx, px, 32), (fn, cn, ky, py, GAL_ROWS)):
+            S = 2 * width + 1 if k else width
+            N = S + 2                                   # points of the region
+            C = (N + 1) // 2 if k else N                # its cells
+            smax, count = (2 * c - 1 if k else c - 1), cells(f, k)
+            for x0 in range(0, c, width):
+                staged = {}
+                for a in range(C):
+                    u = x0 - 1 + a
+                    I, ok = tiles.wrap(u, count, p)
+                    ok = ok and (2 * u if k else u) <= smax + 1
+                    assert not ok or 0 <= I < count
+                    for v in range(2 if k else 1):
+                        x = 2 * a + v if k else a
+                        if x < N:
+                            staged[x] = 2 * I + v if ok and k else I if ok else None
+                assert sorted(staged) == list(range(N))
+                first = 2 * x0 - 2 if k else x0 - 1     # the fine point of region index 0
+                for I in range(x0, min(x0 + width, c)):
+                    lo, hi = (2 * I - 2, 2 * I + 2) if k else (I - 1, I + 1)
+                    for g in range(lo, hi + 1):         # supports and their neighbours
+                        i, ok = tiles.wrap(g, f, p)
+                        if ok:
+                            assert staged[g - first] == i
+                        else:                           # beyond a wall: no point, or one of weight zero
+                            assert staged[g - first] is None or staged[g - first] >= f
 
 
 def smoother_levels(grid):
